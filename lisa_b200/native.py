@@ -1,4 +1,5 @@
-"""Loads ``lib/_lisa_torch.so``: the compiled host side of ``lisa_b200.ops`` (csrc/torch_ops.cpp)."""
+"""``lib/_lisa_torch.so``, the compiled host side of ``lisa_b200.ops`` (csrc/torch_ops.cpp), loaded at the first call: the
+package can be imported, and its build run, before the library exists or while an older one lies in its place."""
 from __future__ import annotations
 
 import importlib.machinery
@@ -23,4 +24,15 @@ def _load():
     return module
 
 
-ext = _load()
+class _Extension:
+    """The module's functions as attributes; the first access loads it and keeps all of them."""
+
+    def __getattr__(self, name):
+        if name.startswith("__"):
+            raise AttributeError(name)
+        module = _load()
+        self.__dict__.update((k, v) for k, v in vars(module).items() if not k.startswith("__"))
+        return getattr(module, name)
+
+
+ext = _Extension()
