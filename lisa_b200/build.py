@@ -81,6 +81,14 @@ def _torch_extension() -> str:
     return TORCH_LIB
 
 
+def _refuse_if_loaded() -> None:
+    """A process that has loaded a library keeps it: built anew under it, its calls would go on running the old code."""
+    cabi = sys.modules.get(f"{os.path.basename(PKG)}._cabi")
+    if cabi is not None and cabi._lib is not None:
+        raise RuntimeError(f"{LIB} is out of date, and this process has already loaded it: build it in a process of its own "
+                           "(`python -m lisa_b200.build`) and start again")
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(LIBDIR, exist_ok=True)
     os.makedirs(OBJDIR, exist_ok=True)
@@ -89,6 +97,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     stamp_file = os.path.join(OBJDIR, "stamp")
     if not force and os.path.exists(LIB) and os.path.exists(TORCH_LIB) and os.path.exists(stamp_file) and open(stamp_file).read() == stamp:
         return LIB
+    _refuse_if_loaded()
     with cf.ThreadPoolExecutor(max_workers=min(8, len(SOURCES))) as ex:
         objs = list(ex.map(lambda s: _compile(s, verbose), SOURCES))
     cmd = [_nvcc(), "-shared", "-o", LIB, *objs, "-gencode", "arch=compute_100a,code=sm_100a", "-cudart", "static"]

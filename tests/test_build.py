@@ -11,11 +11,14 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _compilers(folder):
-    """nvcc and g++ that write a line to the file behind -o and say so; returns the environment that finds them."""
+    """nvcc and g++ that write a line to the file behind -o; returns the environment that finds them.  What links a library copies
+    `$REAL_LIB` instead where that is given, as a new file with a mark at its end."""
     folder.mkdir()
     for name in ("nvcc", "g++"):
         tool = folder / name
-        tool.write_text('#!/bin/sh\nwhile [ "$1" != "-o" ]; do shift; done\necho built > "$2"\n')
+        tool.write_text('#!/bin/sh\nwhile [ "$1" != "-o" ]; do shift; done\n'
+                        'case "$2" in *.so) if [ -n "$REAL_LIB" ]; then cp "$REAL_LIB/$(basename "$2")" "$2.new"; mv "$2.new" "$2"; fi;; esac\n'
+                        'echo built >> "$2"\n')
         tool.chmod(0o755)
     return {**os.environ, "NVCC": str(folder / "nvcc"), "PATH": f"{folder}{os.pathsep}{os.environ['PATH']}", "PYTHONDONTWRITEBYTECODE": "1"}
 
@@ -47,3 +50,35 @@ def test_import_without_a_library_and_a_call_says_what_is_missing(checkout):
                                   "except RuntimeError as e:\n    print('said:', e)")
     assert res.returncode == 0, res.stderr
     assert "said:" in res.stdout and "python -m lisa_b200.build" in res.stdout
+
+
+@pytest.fixture
+def older(checkout, tmp_path):
+    """A checkout with a built library, one of whose sources has changed since; and its environment."""
+    lib = os.path.join(ROOT, "lisa_b200", "lib")
+    if not os.path.exists(os.path.join(lib, "_lisa_torch.so")):
+        pytest.skip("the library is not built")
+    env = {**_compilers(tmp_path / "bin"), "REAL_LIB": lib}
+    res = _python(checkout, "-m", "lisa_b200.build", env=env)
+    assert res.returncode == 0, res.stderr
+    with open(checkout / "lisa_b200" / "csrc" / "api.cu", "a") as f:
+        f.write("// a change\n")
+    return checkout, env
+
+
+def test_entry_point_loads_the_library_that_it_built(older):
+    root, env = older
+    before = os.stat(root / "lisa_b200" / "lib" / "liblisa_cuda.so").st_ino
+    res = _python(root, "-c", "import __graft_entry__ as entry, lisa_b200\nentry.build()\nlisa_b200.native.ext.moe_block\n"
+                              "print(*{line.split()[4] + ' ' + line.split(maxsplit=5)[5].strip() for line in open('/proc/self/maps') if 'lisa_b200/lib' in line}, sep='\\n')", env=env)
+    assert res.returncode == 0, res.stderr
+    mapped = dict(reversed(line.split(maxsplit=1)) for line in res.stdout.splitlines() if "lisa_b200/lib" in line)
+    assert len(mapped) == 2 and not any("deleted" in name for name in mapped), mapped
+    for name, inode in mapped.items():
+        assert os.stat(name).st_ino == int(inode) and (int(inode) != before or "liblisa_cuda" not in name)
+
+
+def test_build_refuses_to_replace_a_loaded_library(older):
+    root, env = older
+    res = _python(root, "-c", "from lisa_b200 import _cabi, build\n_cabi.lib()\nbuild.build()", env=env)
+    assert res.returncode != 0 and "already loaded" in res.stderr, res.stderr
