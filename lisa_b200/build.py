@@ -36,12 +36,19 @@ def _nvcc() -> str:
 
 
 def _stamp(paths) -> str:
+    """What the two libraries are made of: sources, flags, and for the torch extension the torch and Python whose ABI it uses.  The
+    folder of the checkout is left out: a copy of a built tree is built."""
+    import sysconfig
+
+    import torch
+
     h = hashlib.sha256()
     for p in sorted(paths):
         with open(p, "rb") as f:
-            h.update(p.encode())
+            h.update(os.path.relpath(p, ROOT).encode())
             h.update(f.read())
-    h.update(" ".join(NVCC_FLAGS).encode())
+    line = " ".join([*NVCC_FLAGS, torch.__version__, sysconfig.get_config_var("SOABI") or "", *_torch_command()])
+    h.update(line.replace(ROOT, "").encode())
     return h.hexdigest()
 
 
@@ -59,7 +66,7 @@ def _compile(src: str, verbose: bool) -> str:
     return obj
 
 
-def _torch_extension() -> str:
+def _torch_command() -> list[str]:
     """g++ over csrc/torch_ops.cpp against torch's headers; links liblisa_cuda.so from its own folder."""
     import sysconfig
 
@@ -75,7 +82,11 @@ def _torch_extension() -> str:
         cmd += ["-L", path]
     cmd += ["-L", LIBDIR, "-l:liblisa_cuda.so", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
             "-Wl,-rpath,$ORIGIN"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
+    return cmd
+
+
+def _torch_extension() -> str:
+    res = subprocess.run(_torch_command(), capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"g++ failed for {TORCH_SOURCE}:\n{res.stdout}\n{res.stderr}")
     return TORCH_LIB

@@ -82,3 +82,20 @@ def test_build_refuses_to_replace_a_loaded_library(older):
     root, env = older
     res = _python(root, "-c", "from lisa_b200 import _cabi, build\n_cabi.lib()\nbuild.build()", env=env)
     assert res.returncode != 0 and "already loaded" in res.stderr, res.stderr
+
+
+def test_a_copy_of_a_built_tree_is_built(older, tmp_path):
+    root, env = older
+    assert _python(root, "-m", "lisa_b200.build", env=env).returncode == 0
+    shutil.copytree(root, tmp_path / "copy")
+    res = _python(tmp_path / "copy", "-c", "import lisa_b200.build as b\nb._compile = None\nb.build()", env=env)
+    assert res.returncode == 0, res.stderr
+
+
+def test_another_torch_or_compiler_line_builds_anew(older):
+    root, env = older
+    code = ("import torch, lisa_b200.build as b\nb._compile = lambda *a: built.append(a) or '/dev/null'\nbuilt = []\n{}\nb.build()\n"
+            "assert not built, 'built without a change'\n{}\nb.build()\nassert built, 'not built'")
+    for change in ("torch.__version__ += 'x'", "line = b._torch_command()\nb._torch_command = lambda: [*line, '-O1']", "b.NVCC_FLAGS.append('-O2')"):
+        res = _python(root, "-c", code.format("b.build()\nbuilt.clear()", change), env=env)
+        assert res.returncode == 0, res.stderr
