@@ -777,28 +777,43 @@ int lisa_cuda_moe_block(lisa_stream_t stream, const void *x, const float *logits
     if (!workspace || workspace_bytes < lisa_cuda_moe_block_workspace_bytes(tokens, experts, top_k, hidden, inter))
         return fail(LISA_ERR_WORKSPACE, "moe_block: workspace missing or too small");
     if (!aligned16(workspace)) return fail(LISA_ERR_MISALIGNED, "moe_block: workspace must be 16-byte aligned");
+    // Everything is validated before the first launch, by the rules of the calls that the two forms stand for.
+    if (!x || !logits || !out) return fail(LISA_ERR_BAD_ARG, "moe_block: null pointer");
+    if (top_k > experts) return fail(LISA_ERR_BAD_ARG, "moe_block: bad sizes");
+    if (top_k > 32 || experts > 1024) return fail(LISA_ERR_LIMIT, "moe_block: top_k <= 32 and experts <= 1024");
+    if (tokens > (1 << 24)) return fail(LISA_ERR_BAD_ARG, "moe_block: bad token count");
+    const int64_t slots = tokens * top_k;
+    const bool per_slot = slots < decode_slots;
+    const uint32_t *w3[3] = {wg, wu, wd};
+    const void *s3[3] = {sg, su, sd}, *b3[3] = {bg, bu, bd};
+    bool aligned = aligned16(x);
+    for (int i = 0; i < 3; ++i) {
+        const int64_t k = i < 2 ? hidden : inter, n = i < 2 ? inter : hidden;
+        if (per_slot) {
+            if (!w3[i] || !s3[i] || !b3[i]) return fail(LISA_ERR_BAD_ARG, "moe_block: null pointer");
+            LISA_TRY(check_moe_decode("moe_block", experts, k, n, top_k, group_size, bits, dtype));
+            if (!aligned16(x) || !aligned16(w3[i])) return fail(LISA_ERR_MISALIGNED, "moe_block: pointers must be 16-byte aligned");
+        } else {
+            LISA_TRY(check_affine("moe_block", x, slots, k, w3[i], s3[i], b3[i], n, group_size, bits, dtype, out));
+            if (experts * n * k > (1ll << 44)) return fail(LISA_ERR_OVERFLOW, "moe_block: shape too large");
+        }
+        aligned = aligned && aligned16(s3[i]) && aligned16(b3[i]);
+    }
     const MoeBlockPlan plan(tokens, experts, top_k, hidden, inter);
     uint8_t *ws = static_cast<uint8_t *>(workspace);
     int32_t *idx = reinterpret_cast<int32_t *>(ws + plan.idx);
     float *weights = reinterpret_cast<float *>(ws + plan.weights);
-    int rc = lisa_cuda_moe_route(stream, logits, tokens, experts, top_k, idx, weights);
-    if (rc != LISA_OK) return rc;
-    const int64_t slots = tokens * top_k;
-    const uint32_t *w3[3] = {wg, wu, wd};
-    const void *s3[3] = {sg, su, sd}, *b3[3] = {bg, bu, bd};
-    for (int i = 0; i < 3; ++i)
-        LISA_TRY(check_affine("moe_block", x, tokens, i < 2 ? hidden : inter, w3[i], s3[i], b3[i], i < 2 ? inter : hidden, group_size, bits, dtype, out));
-    if (slots < decode_slots && moe_dp_supported(tokens, experts, top_k, hidden, inter, group_size, bits)) {
+    LISA_TRY(moe_route(static_cast<cudaStream_t>(stream), logits, tokens, experts, top_k, idx, weights));
+    if (per_slot && aligned && moe_dp_supported(tokens, experts, top_k, hidden, inter, group_size, bits))
         return moe_dp(static_cast<cudaStream_t>(stream), x, idx, weights, tokens, experts, top_k, hidden, inter, w3, s3, b3, group_size, bits,
                       ws + plan.act, out);
+    if (per_slot) {
+        LISA_TRY(moe_gate_up_act(static_cast<cudaStream_t>(stream), x, idx, nullptr, slots, top_k, experts, hidden, inter, wg, sg, bg, wu, su, bu,
+                                 group_size, bits, ws + plan.act));
+        return moe_down_combine(static_cast<cudaStream_t>(stream), ws + plan.act, idx, weights, tokens, top_k, experts, inter, hidden, wd, sd, bd,
+                                group_size, bits, out);
     }
-    if (slots < decode_slots) {
-        rc = lisa_cuda_moe_gate_up_act(stream, x, idx, nullptr, slots, top_k, experts, hidden, inter, wg, sg, bg, wu, su, bu, group_size,
-                                       bits, dtype, ws + plan.act);
-        if (rc != LISA_OK) return rc;
-        return lisa_cuda_moe_down_combine(stream, ws + plan.act, idx, weights, tokens, top_k, experts, inter, hidden, wd, sd, bd,
-                                          group_size, bits, dtype, out);
-    }
+    int rc = LISA_OK;
     int32_t *sorted_ids = reinterpret_cast<int32_t *>(ws + plan.sorted_ids), *token_rows = reinterpret_cast<int32_t *>(ws + plan.token_rows);
     int32_t *inverse = reinterpret_cast<int32_t *>(ws + plan.inverse);
     if (moe_mm_supported(slots, experts, hidden, inter, group_size, bits)) {

@@ -115,6 +115,31 @@ def test_decode_block_rejections(lib):
     assert gate(slots=0) == _cabi.ERR_BAD_ARG and down(tokens=0) == _cabi.ERR_BAD_ARG
 
 
+def test_moe_block_rejections(lib):
+    """Refused before anything is enqueued: by both forms (decode_slots above and below the eight slots of the call)."""
+    def call(slots_limit, **kw):
+        a = dict(x=16, logits=16, tokens=2, e=8, top_k=4, hidden=256, inter=128, wg=16, sg=16, bg=16, wu=16, su=16, bu=16, wd=16, sd=16, bd=16,
+                 gs=64, bits=4, dtype=0, out=16, ws=16)
+        a.update(kw)
+        need = lib.lisa_cuda_moe_block_workspace_bytes(a["tokens"], a["e"], a["top_k"], a["hidden"], a["inter"])
+        return lib.lisa_cuda_moe_block(None, a["x"], a["logits"], a["tokens"], a["e"], a["top_k"], a["hidden"], a["inter"], a["wg"], a["sg"], a["bg"],
+                                       a["wu"], a["su"], a["bu"], a["wd"], a["sd"], a["bd"], a["gs"], a["bits"], a["dtype"], slots_limit, a["out"],
+                                       a["ws"], a.get("wsb", need))
+    before = lib.lisa_cuda_launch_count()
+    for limit in (0, 32):
+        for name in ("x", "logits", "wg", "wd", "sd", "bu"):
+            assert call(limit, **{name: None}) == _cabi.ERR_BAD_ARG, name
+        assert call(limit, bits=3) == _cabi.ERR_UNSUPPORTED and call(limit, bits=8) == _cabi.ERR_UNSUPPORTED
+        assert call(limit, gs=48) == _cabi.ERR_UNSUPPORTED
+        assert call(limit, dtype=1) == _cabi.ERR_UNSUPPORTED
+        assert call(limit, x=8) == _cabi.ERR_MISALIGNED and call(limit, wd=24) == _cabi.ERR_MISALIGNED
+        assert call(limit, top_k=9) == _cabi.ERR_BAD_ARG            # more than the experts
+        assert call(limit, e=2048) == _cabi.ERR_LIMIT
+        assert call(limit, e=1024, hidden=1 << 18, inter=1 << 17) == _cabi.ERR_OVERFLOW  # experts * n * k
+        assert call(limit, ws=None) == _cabi.ERR_WORKSPACE and call(limit, wsb=64) == _cabi.ERR_WORKSPACE
+    assert lib.lisa_cuda_launch_count() == before
+
+
 def test_addnorm_rejections(lib):
     import ctypes as C
     one = (C.c_void_p * 1)(16)
