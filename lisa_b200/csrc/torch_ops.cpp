@@ -422,14 +422,30 @@ PyObject *moe_block(PyObject *, Args a, Py_ssize_t na) {
         Linears l;
         for (int i = 0; i < 3; ++i) l.add(a[2 + 3 * i], a[3 + 3 * i], a[4 + 3 * i]);
         const at::Tensor xc = whole(x), logits = whole(lg.scalar_type() == at::kFloat ? lg : lg.to(at::kFloat));
+        const int64_t gs = integer(a[11]), bits = integer(a[12]);
+        for (int i = 0; i < 3; ++i)
+            for (const at::Tensor &t : l.keep[i])
+                if (t.dim() != 3) refuse(LISA_ERR_BAD_ARG, "moe_block: weights, scales and biases have three dimensions: experts, rows, columns");
+        if (logits.dim() != 2 || x.dim() < 1) refuse(LISA_ERR_BAD_ARG, "moe_block: shapes of x, the logits and the experts disagree");
         const int64_t tokens = logits.size(0), hidden = x.size(-1), experts = l.keep[0][0].size(0), inter = l.keep[0][0].size(1);
-        if (logits.dim() != 2 || logits.size(1) != experts || xc.numel() != tokens * hidden) refuse(LISA_ERR_BAD_ARG, "moe_block: shapes of x, the logits and the experts disagree");
+        if (logits.size(1) != experts || xc.numel() != tokens * hidden) refuse(LISA_ERR_BAD_ARG, "moe_block: shapes of x, the logits and the experts disagree");
+        if (bits < 1 || bits > 32 || gs < 1) refuse(LISA_ERR_UNSUPPORTED, "moe_block: bits must be 2 or 4");
+        // the kernels take every size from here: each tensor has to have it
+        for (int i = 0; i < 3; ++i) {
+            const int64_t n = i < 2 ? inter : hidden, k = i < 2 ? hidden : inter;
+            const at::Tensor &w = l.keep[i][0], &sc = l.keep[i][1], &bi = l.keep[i][2];
+            if (w.size(0) != experts || w.size(1) != n || w.size(2) * 32 != k * bits || sc.size(0) != experts || sc.size(1) != n || sc.size(2) * gs != k ||
+                bi.sizes() != sc.sizes())
+                refuse(LISA_ERR_BAD_ARG, i == 0 ? "moe_block: shapes of the gate projection, its scales and biases disagree with x and the logits"
+                                       : i == 1 ? "moe_block: shapes of the up projection, its scales and biases disagree with the gate's"
+                                                : "moe_block: shapes of the down projection, its scales and biases disagree with the gate's");
+            if (sc.element_size() != 2 || bi.element_size() != 2) refuse(LISA_ERR_BAD_ARG, "moe_block: scales and biases must be 16-bit");
+        }
         const int top_k = static_cast<int>(integer(a[13]));
         const size_t need = lisa_cuda_moe_block_workspace_bytes(tokens, experts, top_k, hidden, inter);
-        const at::Tensor ws = empty({static_cast<int64_t>(need)}, at::kByte, x), out = empty({tokens, l.keep[2][0].size(1)}, x);
-        if (out.size(1) != hidden) refuse(LISA_ERR_BAD_ARG, "moe_block: the down projection's rows are not the hidden size");
+        const at::Tensor ws = empty({static_cast<int64_t>(need)}, at::kByte, x), out = empty({tokens, hidden}, x);
         check(lisa_cuda_moe_block(stream_of(Py_None), ptr(xc), ptr_of<float>(logits), tokens, experts, top_k, hidden, inter, l.w[0], l.s[0], l.b[0],
-                                  l.w[1], l.s[1], l.b[1], l.w[2], l.s[2], l.b[2], static_cast<int>(integer(a[11])), static_cast<int>(integer(a[12])),
+                                  l.w[1], l.s[1], l.b[1], l.w[2], l.s[2], l.b[2], static_cast<int>(gs), static_cast<int>(bits),
                                   dtype_code(xc), integer(a[14]), out_ptr(out), out_ptr(ws), need));
         return wrap(out);
     });
