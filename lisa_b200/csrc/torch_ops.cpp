@@ -7,6 +7,7 @@
 // (include/lisa_cuda.h).  Each function raises the LisaError that the Python form raised.
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -67,17 +68,40 @@ bool truth(PyObject *o) {
     if (v < 0) throw PythonFailure{};
     return v != 0;
 }
-// None: the current stream; else an object with a `cuda_stream`, or the handle itself.
-lisa_stream_t stream_of(PyObject *o) {
-    if (o == Py_None) return c10::cuda::getCurrentCUDAStream().stream();
-    if (PyObject *h = PyObject_GetAttrString(o, "cuda_stream")) {
-        const int64_t v = integer(h);
-        Py_DECREF(h);
-        return reinterpret_cast<lisa_stream_t>(v);
-    }
-    PyErr_Clear();
-    return reinterpret_cast<lisa_stream_t>(integer(o));
+at::Tensor empty(at::IntArrayRef size, at::ScalarType dtype, const at::Tensor &like) {
+    return at::detail::empty_cuda(size, dtype, like.device(), std::nullopt);
 }
+at::Tensor empty(at::IntArrayRef size, const at::Tensor &like) { return empty(size, like.scalar_type(), like); }
+// The stream of a call: None: the current one; else an object with a `cuda_stream`, or the handle itself.  While this lives, tensors are
+// allocated and copied on that stream, so that what ends with the call (contiguous copies, workspaces) goes back to the pool of
+// the stream that still reads it.  Outputs belong to the caller's current stream (`output`).
+class CallStream {
+  public:
+    explicit CallStream(PyObject *o) : caller_(c10::cuda::getCurrentCUDAStream()), handle_(caller_.stream()) {
+        if (o == Py_None) return;
+        if (PyObject *h = PyObject_GetAttrString(o, "cuda_stream")) {
+            handle_ = handle(h);
+            Py_DECREF(h);
+        } else {
+            PyErr_Clear();
+            handle_ = handle(o);
+        }
+        if (handle_ != caller_.stream()) guard_.reset_stream(c10::cuda::getStreamFromExternal(handle_, caller_.device_index()));
+    }
+    operator lisa_stream_t() const { return handle_; }
+    at::Tensor output(at::IntArrayRef size, at::ScalarType dtype, const at::Tensor &like) const {
+        c10::cuda::OptionalCUDAStreamGuard back;
+        if (handle_ != caller_.stream()) back.reset_stream(caller_);
+        return empty(size, dtype, like);
+    }
+    at::Tensor output(at::IntArrayRef size, const at::Tensor &like) const { return output(size, like.scalar_type(), like); }
+
+  private:
+    static cudaStream_t handle(PyObject *o) { return reinterpret_cast<cudaStream_t>(integer(o)); }
+    c10::cuda::CUDAStream caller_;
+    cudaStream_t handle_;
+    c10::cuda::OptionalCUDAStreamGuard guard_;
+};
 int dtype_code(const at::Tensor &t) {
     switch (t.scalar_type()) {
         case at::kBFloat16: return LISA_BF16;
@@ -92,10 +116,6 @@ at::Tensor words(const at::Tensor &w) {
         throw LisaFailure{LISA_ERR_BAD_ARG, "packed weights must be uint32 words, got torch." + std::string(c10::toString(w.scalar_type()))};
     return whole(w);
 }
-at::Tensor empty(at::IntArrayRef size, at::ScalarType dtype, const at::Tensor &like) {
-    return at::detail::empty_cuda(size, dtype, like.device(), std::nullopt);
-}
-at::Tensor empty(at::IntArrayRef size, const at::Tensor &like) { return empty(size, like.scalar_type(), like); }
 const void *ptr(const at::Tensor &t) { return t.defined() ? t.const_data_ptr() : nullptr; }
 void *out_ptr(const at::Tensor &t) { return t.defined() ? t.mutable_data_ptr() : nullptr; }
 template <typename T>
@@ -212,12 +232,13 @@ PyObject *quantized_matmul(PyObject *, Args a, Py_ssize_t na) {
         need_cuda(w0);
         need_cuda(s0);
         need_cuda(b0);
+        const CallStream stream(a[7]);
         const int64_t k = x.size(-1), m = rows_of(x, k), gs = integer(a[5]), bits = integer(a[6]);
         const at::Tensor xc = whole(x), w = words(w0), s = whole(s0), b = whole(b0);
         const int64_t n = w.size(0);
         if (bits <= 0 || w.size(-1) * 32 / bits != k || s.size(-1) * gs != k) refuse(LISA_ERR_BAD_ARG, "quantized_matmul: shapes of x, w and scales disagree");
-        const at::Tensor y = out.defined() ? out : empty(with_last(x, n), x);
-        check(lisa_cuda_quantized_matmul_ex(stream_of(a[7]), ptr(xc), m, k, ptr_of<uint32_t>(w), ptr(s), ptr(b), n, truth(a[4]), static_cast<int>(gs),
+        const at::Tensor y = out.defined() ? out : stream.output(with_last(x, n), x);
+        check(lisa_cuda_quantized_matmul_ex(stream, ptr(xc), m, k, ptr_of<uint32_t>(w), ptr(s), ptr(b), n, truth(a[4]), static_cast<int>(gs),
                                             static_cast<int>(bits), dtype_code(xc), out_ptr(y), static_cast<unsigned>(integer(a[9]))));
         return wrap(out.defined() ? y.reshape(with_last(x, n)) : y);
     });
@@ -228,16 +249,17 @@ PyObject *quantized_matmul_siblings(PyObject *, Args a, Py_ssize_t na) {
     return guarded(na, 7, [&]() -> PyObject * {
         const at::Tensor &x = tensor(a[0]);
         need_cuda(x);
+        const CallStream stream(a[5]);
         const int64_t k = x.size(-1), m = rows_of(x, k), gs = integer(a[3]), bits = integer(a[4]);
         const at::Tensor xc = whole(x);
         Linears l;
         l.read(a[1]);
         for (int i = 0; i < l.count; ++i) {
             l.fit(i, k, gs, bits, "quantized_matmul_siblings: shapes of x, w and scales disagree");
-            l.y[i] = empty(with_last(x, l.n[i]), x);
+            l.y[i] = stream.output(with_last(x, l.n[i]), x);
             l.out[i] = out_ptr(l.y[i]);
         }
-        check(lisa_cuda_quantized_matmul_siblings(stream_of(a[5]), ptr(xc), m, k, l.count, l.w, l.s, l.b, l.n, truth(a[2]), static_cast<int>(gs),
+        check(lisa_cuda_quantized_matmul_siblings(stream, ptr(xc), m, k, l.count, l.w, l.s, l.b, l.n, truth(a[2]), static_cast<int>(gs),
                                                   static_cast<int>(bits), dtype_code(xc), l.out, static_cast<unsigned>(integer(a[6]))));
         return list_of(l.y, l.count);
     });
@@ -250,6 +272,7 @@ PyObject *quantized_matmul_addnorm(PyObject *, Args a, Py_ssize_t na) {
         need_cuda(x);
         need_cuda(r);
         need_cuda(nw);
+        const CallStream stream(a[8]);
         const int64_t k = x.size(-1), m = rows_of(x, k), gs = integer(a[5]), bits = integer(a[6]);
         const at::Tensor xc = whole(x), rc = whole(r), nc = whole(nw);
         if (rc.numel() != xc.numel()) throw std::runtime_error("shape '" + std::to_string(m) + " x " + std::to_string(k) + "' is invalid for the residual");
@@ -257,11 +280,11 @@ PyObject *quantized_matmul_addnorm(PyObject *, Args a, Py_ssize_t na) {
         l.read(a[4]);
         for (int i = 0; i < l.count; ++i) {
             l.fit(i, k, gs, bits, "quantized_matmul_addnorm: shapes of x, w and scales disagree");
-            l.y[i] = empty(with_last(x, l.n[i]), x);
+            l.y[i] = stream.output(with_last(x, l.n[i]), x);
             l.out[i] = out_ptr(l.y[i]);
         }
-        const at::Tensor total = empty(x.sizes(), x), normed = truth(a[7]) ? empty(x.sizes(), x) : at::Tensor();
-        check(lisa_cuda_quantized_matmul_addnorm(stream_of(a[8]), ptr(xc), ptr(rc), ptr(nc), static_cast<float>(real(a[3])), m, k, l.count, l.w, l.s, l.b,
+        const at::Tensor total = stream.output(x.sizes(), x), normed = truth(a[7]) ? stream.output(x.sizes(), x) : at::Tensor();
+        check(lisa_cuda_quantized_matmul_addnorm(stream, ptr(xc), ptr(rc), ptr(nc), static_cast<float>(real(a[3])), m, k, l.count, l.w, l.s, l.b,
                                                  l.n, 1, static_cast<int>(gs), static_cast<int>(bits), dtype_code(xc), l.out, out_ptr(total),
                                                  out_ptr(normed), static_cast<unsigned>(integer(a[9]))));
         return tuple_of({list_of(l.y, l.count), wrap(total), wrap(normed)});
@@ -274,15 +297,17 @@ PyObject *quantized_matmul_swiglu(PyObject *, Args a, Py_ssize_t na) {
         const at::Tensor &g = tensor(a[0]), &u = tensor(a[1]);
         need_cuda(g);
         need_cuda(u);
+        const CallStream stream(a[8]);
         const int64_t k = g.size(-1), m = rows_of(g, k), gs = integer(a[5]), bits = integer(a[6]);
         const at::Tensor gc = whole(g), uc = whole(u);
         if (uc.numel() != gc.numel()) throw std::runtime_error("swiglu: gate and up differ in size");
         Linears l;
         l.add(a[2], a[3], a[4]);
-        const at::Tensor y = empty(with_last(g, l.n[0]), g), act = truth(a[7]) ? empty(g.sizes(), g) : at::Tensor();
-        // decode rows: a place for the activation, so that the library may form it once (shapes that need one are still refused)
+        const at::Tensor y = stream.output(with_last(g, l.n[0]), g), act = truth(a[7]) ? stream.output(g.sizes(), g) : at::Tensor();
+        // decode rows: a place for the activation, so that the library may form it once (rows too long for the one-launch kernels then run as
+        // two steps)
         const at::Tensor scratch = !act.defined() && m > 2 && m <= 8 && gs == 64 && bits != 8 ? empty(g.sizes(), g) : act;
-        check(lisa_cuda_quantized_matmul_swiglu(stream_of(a[8]), ptr(gc), ptr(uc), m, k, l.w[0], l.s[0], l.b[0], l.n[0], 1, static_cast<int>(gs),
+        check(lisa_cuda_quantized_matmul_swiglu(stream, ptr(gc), ptr(uc), m, k, l.w[0], l.s[0], l.b[0], l.n[0], 1, static_cast<int>(gs),
                                                 static_cast<int>(bits), dtype_code(gc), out_ptr(y), out_ptr(scratch), static_cast<unsigned>(integer(a[9]))));
         return tuple_of({wrap(y), wrap(act)});
     });
@@ -292,9 +317,10 @@ PyObject *quantized_matmul_swiglu(PyObject *, Args a, Py_ssize_t na) {
 PyObject *dequantize_rows(PyObject *, Args a, Py_ssize_t na) {
     return guarded(na, 7, [&]() -> PyObject * {
         const at::Tensor &ids = tensor(a[3]);
+        need_cuda(ids);
+        const CallStream stream(a[6]);
         Linears l;
         l.add(a[0], a[1], a[2]);
-        need_cuda(ids);
         const int64_t gs = integer(a[4]), bits = integer(a[5]);
         if (bits <= 0) refuse(LISA_ERR_UNSUPPORTED, "dequantize_rows: bits must be 2, 4 or 8");
         const at::Tensor &s = l.keep[0][1];
@@ -302,8 +328,8 @@ PyObject *dequantize_rows(PyObject *, Args a, Py_ssize_t na) {
         const at::Tensor flat = whole(ids.scalar_type() == at::kInt ? ids : ids.to(at::kInt));
         c10::SmallVector<int64_t, 5> size(ids.sizes().begin(), ids.sizes().end());
         size.push_back(k);
-        const at::Tensor out = empty(size, s);
-        check(lisa_cuda_dequantize_rows(stream_of(a[6]), l.w[0], l.s[0], l.b[0], ptr_of<int32_t>(flat), flat.numel(), l.n[0], k, static_cast<int>(gs),
+        const at::Tensor out = stream.output(size, s);
+        check(lisa_cuda_dequantize_rows(stream, l.w[0], l.s[0], l.b[0], ptr_of<int32_t>(flat), flat.numel(), l.n[0], k, static_cast<int>(gs),
                                         static_cast<int>(bits), dtype_code(s), out_ptr(out)));
         return wrap(out);
     });
@@ -315,6 +341,7 @@ PyObject *packed_matvec(PyObject *, Args a, Py_ssize_t na) {
         const at::Tensor &w = tensor(a[1]), &x = tensor(a[2]);
         need_cuda(w);
         need_cuda(x);
+        const CallStream stream(a[3]);
         const int code = static_cast<int>(integer(a[0]));
         if (w.dim() != 2 || w.scalar_type() != at::kByte || !w.is_contiguous()) refuse(LISA_ERR_BAD_ARG, "unsupported GGUF quantized matvec layout");
         if (x.dim() != 2 || x.scalar_type() != at::kFloat) refuse(LISA_ERR_BAD_ARG, "invalid GGUF matvec input rows");
@@ -322,8 +349,8 @@ PyObject *packed_matvec(PyObject *, Args a, Py_ssize_t na) {
         const int64_t block = code == LISA_GGUF_Q2_K ? 84 : code == LISA_GGUF_Q4_K ? 144 : code == LISA_GGUF_Q5_K ? 176 : 0;
         if (block && row_bytes % block == 0 && x.size(1) != row_bytes / block * 256)
             refuse(LISA_ERR_BAD_ARG, "GGUF matvec input width does not match the packed rows");
-        const at::Tensor xc = whole(x), y = empty({tokens, rows}, x);
-        check(lisa_cuda_gguf_packed_matvec(stream_of(a[3]), code, ptr_of<uint8_t>(w), rows, row_bytes, ptr_of<float>(xc), tokens, out_of<float>(y)));
+        const at::Tensor xc = whole(x), y = stream.output({tokens, rows}, x);
+        check(lisa_cuda_gguf_packed_matvec(stream, code, ptr_of<uint8_t>(w), rows, row_bytes, ptr_of<float>(xc), tokens, out_of<float>(y)));
         return wrap(y);
     });
 }
@@ -335,14 +362,15 @@ PyObject *packed_matmul(PyObject *, Args a, Py_ssize_t na) {
         at::Tensor ws = tensor(a[3], true);
         need_cuda(w);
         need_cuda(x);
+        const CallStream stream(a[4]);
         const int code = static_cast<int>(integer(a[0]));
         if (w.dim() != 2 || w.scalar_type() != at::kByte || !w.is_contiguous()) refuse(LISA_ERR_BAD_ARG, "unsupported GGUF quantized matvec layout");
         if (x.dim() != 2 || x.scalar_type() != at::kFloat) refuse(LISA_ERR_BAD_ARG, "invalid GGUF matvec input rows");
         const int64_t rows = w.size(0), row_bytes = w.size(1), tokens = x.size(0);
         const size_t need = lisa_cuda_gguf_packed_matmul_workspace_bytes(tokens, row_bytes, code);
         if (!ws.defined() && need) ws = empty({static_cast<int64_t>(need)}, at::kByte, x);
-        const at::Tensor xc = whole(x), y = empty({tokens, rows}, x);
-        check(lisa_cuda_gguf_packed_matmul(stream_of(a[4]), code, ptr_of<uint8_t>(w), rows, row_bytes, ptr_of<float>(xc), tokens, out_of<float>(y),
+        const at::Tensor xc = whole(x), y = stream.output({tokens, rows}, x);
+        check(lisa_cuda_gguf_packed_matmul(stream, code, ptr_of<uint8_t>(w), rows, row_bytes, ptr_of<float>(xc), tokens, out_of<float>(y),
                                            out_ptr(ws), ws.defined() ? static_cast<size_t>(ws.numel()) : 0));
         return wrap(y);
     });
@@ -355,13 +383,14 @@ PyObject *expert_matvec(PyObject *, Args a, Py_ssize_t na) {
         need_cuda(w);
         need_cuda(x);
         need_cuda(ids);
+        const CallStream stream(a[4]);
         const int code = static_cast<int>(integer(a[0]));
         if (w.dim() != 3 || w.scalar_type() != at::kByte || !w.is_contiguous()) refuse(LISA_ERR_BAD_ARG, "unsupported GGUF quantized matvec layout");
         if (ids.dim() != 2 || ids.scalar_type() != at::kInt || x.dim() != 3 || x.scalar_type() != at::kFloat || x.size(0) != ids.size(0))
             refuse(LISA_ERR_BAD_ARG, "invalid GGUF expert matvec geometry");
         const int64_t tokens = ids.size(0), top_k = ids.size(1), rows = w.size(1);
-        const at::Tensor xc = whole(x), ic = whole(ids), y = empty({tokens, top_k, rows}, x);
-        check(lisa_cuda_gguf_expert_matvec(stream_of(a[4]), code, ptr_of<uint8_t>(w), w.size(0), rows, w.size(2), ptr_of<float>(xc), tokens, x.size(1),
+        const at::Tensor xc = whole(x), ic = whole(ids), y = stream.output({tokens, top_k, rows}, x);
+        check(lisa_cuda_gguf_expert_matvec(stream, code, ptr_of<uint8_t>(w), w.size(0), rows, w.size(2), ptr_of<float>(xc), tokens, x.size(1),
                                            ptr_of<int32_t>(ic), top_k, out_of<float>(y)));
         return wrap(y);
     });
@@ -373,13 +402,14 @@ PyObject *gather_qmm(PyObject *, Args a, Py_ssize_t na) {
         const at::Tensor &x = tensor(a[0]), &w0 = tensor(a[1]), &s0 = tensor(a[2]), &b0 = tensor(a[3], true), &lhs = tensor(a[4], true), &rhs = tensor(a[5], true);
         at::Tensor ws = tensor(a[11], true);
         for (const at::Tensor *t : {&x, &w0, &s0, &b0, &rhs}) need_cuda(*t);
+        const CallStream stream(a[10]);
         const int64_t k = x.size(-1), rows = rows_of(x, k), experts = w0.size(0), n = w0.size(-2);
         const at::Tensor xc = whole(x), w = words(w0), s = whole(s0), b = whole(b0);
-        const at::Tensor y = empty(with_last(x, n), x);
+        const at::Tensor y = stream.output(with_last(x, n), x);
         const size_t need = lisa_cuda_gather_qmm_workspace_bytes(rows, experts);
         if (!ws.defined() && need) ws = empty({static_cast<int64_t>(need)}, at::kByte, x);
         const at::Tensor ids = !rhs.defined() ? rhs : whole(rhs.scalar_type() == at::kInt ? rhs : rhs.to(at::kInt));
-        check(lisa_cuda_gather_qmm(stream_of(a[10]), ptr(xc), rows, k, ptr_of<uint32_t>(w), ptr(s), ptr(b), ptr_of<int32_t>(lhs), ptr_of<int32_t>(ids),
+        check(lisa_cuda_gather_qmm(stream, ptr(xc), rows, k, ptr_of<uint32_t>(w), ptr(s), ptr(b), ptr_of<int32_t>(lhs), ptr_of<int32_t>(ids),
                                    experts, n, truth(a[6]), static_cast<int>(integer(a[7])), static_cast<int>(integer(a[8])), truth(a[9]),
                                    dtype_code(xc), out_ptr(y), out_ptr(ws), ws.defined() ? static_cast<size_t>(ws.numel()) : 0));
         return wrap(y);
@@ -393,6 +423,7 @@ PyObject *gather_qmm_siblings(PyObject *, Args a, Py_ssize_t na) {
         at::Tensor ws = tensor(a[6], true);
         need_cuda(x);
         need_cuda(rhs);
+        const CallStream stream(a[5]);
         const int64_t k = x.size(-1), rows = rows_of(x, k);
         const at::Tensor xc = whole(x), ids = whole(rhs.scalar_type() == at::kInt ? rhs : rhs.to(at::kInt));
         Linears l;
@@ -401,12 +432,12 @@ PyObject *gather_qmm_siblings(PyObject *, Args a, Py_ssize_t na) {
         const int64_t experts = l.keep[0][0].size(0), n = l.keep[0][0].size(-2);
         for (int i = 0; i < l.count; ++i) {
             if (l.keep[i][0].size(0) != experts || l.keep[i][0].size(-2) != n) refuse(LISA_ERR_BAD_ARG, "gather_qmm_siblings: the linears must have one shape");
-            l.y[i] = empty(with_last(x, n), x);
+            l.y[i] = stream.output(with_last(x, n), x);
             l.out[i] = out_ptr(l.y[i]);
         }
         const size_t need = lisa_cuda_gather_qmm_workspace_bytes(rows, experts);
         if (!ws.defined() && need) ws = empty({static_cast<int64_t>(need)}, at::kByte, x);
-        check(lisa_cuda_gather_qmm_siblings(stream_of(a[5]), ptr(xc), rows, k, l.count, l.w, l.s, l.b, ptr_of<int32_t>(ids), experts, n, 1,
+        check(lisa_cuda_gather_qmm_siblings(stream, ptr(xc), rows, k, l.count, l.w, l.s, l.b, ptr_of<int32_t>(ids), experts, n, 1,
                                             static_cast<int>(integer(a[3])), static_cast<int>(integer(a[4])), 1, dtype_code(xc), l.out, out_ptr(ws),
                                             ws.defined() ? static_cast<size_t>(ws.numel()) : 0));
         return list_of(l.y, l.count);
@@ -444,7 +475,7 @@ PyObject *moe_block(PyObject *, Args a, Py_ssize_t na) {
         const int top_k = static_cast<int>(integer(a[13]));
         const size_t need = lisa_cuda_moe_block_workspace_bytes(tokens, experts, top_k, hidden, inter);
         const at::Tensor ws = empty({static_cast<int64_t>(need)}, at::kByte, x), out = empty({tokens, hidden}, x);
-        check(lisa_cuda_moe_block(stream_of(Py_None), ptr(xc), ptr_of<float>(logits), tokens, experts, top_k, hidden, inter, l.w[0], l.s[0], l.b[0],
+        check(lisa_cuda_moe_block(c10::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr_of<float>(logits), tokens, experts, top_k, hidden, inter, l.w[0], l.s[0], l.b[0],
                                   l.w[1], l.s[1], l.b[1], l.w[2], l.s[2], l.b[2], static_cast<int>(gs), static_cast<int>(bits),
                                   dtype_code(xc), integer(a[14]), out_ptr(out), out_ptr(ws), need));
         return wrap(out);
