@@ -31,6 +31,21 @@ struct PythonFailure {};  // a Python exception is already set
 void check(int rc) {
     if (rc != LISA_OK) throw LisaFailure{rc, lisa_cuda_last_error_string()};
 }
+// A call of the library without the interpreter's lock: where a stream's queue is full a launch waits, and other threads (among them
+// those that such a stream may be waiting for) go on.
+template <typename F>
+void enqueue(F &&call) {
+    struct Unlocked {
+        PyThreadState *state = PyEval_SaveThread();
+        ~Unlocked() { PyEval_RestoreThread(state); }
+    };
+    int rc;
+    {
+        Unlocked here;
+        rc = call();
+    }
+    check(rc);
+}
 
 // A tensor argument; `optional` lets None through as an undefined tensor.
 const at::Tensor &tensor(PyObject *o, bool optional = false) {
@@ -238,8 +253,12 @@ PyObject *quantized_matmul(PyObject *, Args a, Py_ssize_t na) {
         const int64_t n = w.size(0);
         if (bits <= 0 || w.size(-1) * 32 / bits != k || s.size(-1) * gs != k) refuse(LISA_ERR_BAD_ARG, "quantized_matmul: shapes of x, w and scales disagree");
         const at::Tensor y = out.defined() ? out : stream.output(with_last(x, n), x);
-        check(lisa_cuda_quantized_matmul_ex(stream, ptr(xc), m, k, ptr_of<uint32_t>(w), ptr(s), ptr(b), n, truth(a[4]), static_cast<int>(gs),
-                                            static_cast<int>(bits), dtype_code(xc), out_ptr(y), static_cast<unsigned>(integer(a[9]))));
+        const int transpose = truth(a[4]);
+        const unsigned flags = static_cast<unsigned>(integer(a[9]));
+        enqueue([&] {
+            return lisa_cuda_quantized_matmul_ex(stream, ptr(xc), m, k, ptr_of<uint32_t>(w), ptr(s), ptr(b), n, transpose, static_cast<int>(gs),
+                                            static_cast<int>(bits), dtype_code(xc), out_ptr(y), flags);
+        });
         return wrap(out.defined() ? y.reshape(with_last(x, n)) : y);
     });
 }
@@ -259,8 +278,12 @@ PyObject *quantized_matmul_siblings(PyObject *, Args a, Py_ssize_t na) {
             l.y[i] = stream.output(with_last(x, l.n[i]), x);
             l.out[i] = out_ptr(l.y[i]);
         }
-        check(lisa_cuda_quantized_matmul_siblings(stream, ptr(xc), m, k, l.count, l.w, l.s, l.b, l.n, truth(a[2]), static_cast<int>(gs),
-                                                  static_cast<int>(bits), dtype_code(xc), l.out, static_cast<unsigned>(integer(a[6]))));
+        const int transpose = truth(a[2]);
+        const unsigned flags = static_cast<unsigned>(integer(a[6]));
+        enqueue([&] {
+            return lisa_cuda_quantized_matmul_siblings(stream, ptr(xc), m, k, l.count, l.w, l.s, l.b, l.n, transpose, static_cast<int>(gs),
+                                                  static_cast<int>(bits), dtype_code(xc), l.out, flags);
+        });
         return list_of(l.y, l.count);
     });
 }
@@ -284,9 +307,13 @@ PyObject *quantized_matmul_addnorm(PyObject *, Args a, Py_ssize_t na) {
             l.out[i] = out_ptr(l.y[i]);
         }
         const at::Tensor total = stream.output(x.sizes(), x), normed = truth(a[7]) ? stream.output(x.sizes(), x) : at::Tensor();
-        check(lisa_cuda_quantized_matmul_addnorm(stream, ptr(xc), ptr(rc), ptr(nc), static_cast<float>(real(a[3])), m, k, l.count, l.w, l.s, l.b,
+        const unsigned flags = static_cast<unsigned>(integer(a[9]));
+        const float eps = static_cast<float>(real(a[3]));
+        enqueue([&] {
+            return lisa_cuda_quantized_matmul_addnorm(stream, ptr(xc), ptr(rc), ptr(nc), eps, m, k, l.count, l.w, l.s, l.b,
                                                  l.n, 1, static_cast<int>(gs), static_cast<int>(bits), dtype_code(xc), l.out, out_ptr(total),
-                                                 out_ptr(normed), static_cast<unsigned>(integer(a[9]))));
+                                                 out_ptr(normed), flags);
+        });
         return tuple_of({list_of(l.y, l.count), wrap(total), wrap(normed)});
     });
 }
@@ -307,8 +334,11 @@ PyObject *quantized_matmul_swiglu(PyObject *, Args a, Py_ssize_t na) {
         // decode rows: a place for the activation, so that the library may form it once (rows too long for the one-launch kernels then run as
         // two steps)
         const at::Tensor scratch = !act.defined() && m > 2 && m <= 8 && gs == 64 && bits != 8 ? empty(g.sizes(), g) : act;
-        check(lisa_cuda_quantized_matmul_swiglu(stream, ptr(gc), ptr(uc), m, k, l.w[0], l.s[0], l.b[0], l.n[0], 1, static_cast<int>(gs),
-                                                static_cast<int>(bits), dtype_code(gc), out_ptr(y), out_ptr(scratch), static_cast<unsigned>(integer(a[9]))));
+        const unsigned flags = static_cast<unsigned>(integer(a[9]));
+        enqueue([&] {
+            return lisa_cuda_quantized_matmul_swiglu(stream, ptr(gc), ptr(uc), m, k, l.w[0], l.s[0], l.b[0], l.n[0], 1, static_cast<int>(gs),
+                                                static_cast<int>(bits), dtype_code(gc), out_ptr(y), out_ptr(scratch), flags);
+        });
         return tuple_of({wrap(y), wrap(act)});
     });
 }
@@ -329,8 +359,10 @@ PyObject *dequantize_rows(PyObject *, Args a, Py_ssize_t na) {
         c10::SmallVector<int64_t, 5> size(ids.sizes().begin(), ids.sizes().end());
         size.push_back(k);
         const at::Tensor out = stream.output(size, s);
-        check(lisa_cuda_dequantize_rows(stream, l.w[0], l.s[0], l.b[0], ptr_of<int32_t>(flat), flat.numel(), l.n[0], k, static_cast<int>(gs),
-                                        static_cast<int>(bits), dtype_code(s), out_ptr(out)));
+        enqueue([&] {
+            return lisa_cuda_dequantize_rows(stream, l.w[0], l.s[0], l.b[0], ptr_of<int32_t>(flat), flat.numel(), l.n[0], k, static_cast<int>(gs),
+                                        static_cast<int>(bits), dtype_code(s), out_ptr(out));
+        });
         return wrap(out);
     });
 }
@@ -350,7 +382,9 @@ PyObject *packed_matvec(PyObject *, Args a, Py_ssize_t na) {
         if (block && row_bytes % block == 0 && x.size(1) != row_bytes / block * 256)
             refuse(LISA_ERR_BAD_ARG, "GGUF matvec input width does not match the packed rows");
         const at::Tensor xc = whole(x), y = stream.output({tokens, rows}, x);
-        check(lisa_cuda_gguf_packed_matvec(stream, code, ptr_of<uint8_t>(w), rows, row_bytes, ptr_of<float>(xc), tokens, out_of<float>(y)));
+        enqueue([&] {
+            return lisa_cuda_gguf_packed_matvec(stream, code, ptr_of<uint8_t>(w), rows, row_bytes, ptr_of<float>(xc), tokens, out_of<float>(y));
+        });
         return wrap(y);
     });
 }
@@ -370,8 +404,10 @@ PyObject *packed_matmul(PyObject *, Args a, Py_ssize_t na) {
         const size_t need = lisa_cuda_gguf_packed_matmul_workspace_bytes(tokens, row_bytes, code);
         if (!ws.defined() && need) ws = empty({static_cast<int64_t>(need)}, at::kByte, x);
         const at::Tensor xc = whole(x), y = stream.output({tokens, rows}, x);
-        check(lisa_cuda_gguf_packed_matmul(stream, code, ptr_of<uint8_t>(w), rows, row_bytes, ptr_of<float>(xc), tokens, out_of<float>(y),
-                                           out_ptr(ws), ws.defined() ? static_cast<size_t>(ws.numel()) : 0));
+        enqueue([&] {
+            return lisa_cuda_gguf_packed_matmul(stream, code, ptr_of<uint8_t>(w), rows, row_bytes, ptr_of<float>(xc), tokens, out_of<float>(y),
+                                           out_ptr(ws), ws.defined() ? static_cast<size_t>(ws.numel()) : 0);
+        });
         return wrap(y);
     });
 }
@@ -390,8 +426,10 @@ PyObject *expert_matvec(PyObject *, Args a, Py_ssize_t na) {
             refuse(LISA_ERR_BAD_ARG, "invalid GGUF expert matvec geometry");
         const int64_t tokens = ids.size(0), top_k = ids.size(1), rows = w.size(1);
         const at::Tensor xc = whole(x), ic = whole(ids), y = stream.output({tokens, top_k, rows}, x);
-        check(lisa_cuda_gguf_expert_matvec(stream, code, ptr_of<uint8_t>(w), w.size(0), rows, w.size(2), ptr_of<float>(xc), tokens, x.size(1),
-                                           ptr_of<int32_t>(ic), top_k, out_of<float>(y)));
+        enqueue([&] {
+            return lisa_cuda_gguf_expert_matvec(stream, code, ptr_of<uint8_t>(w), w.size(0), rows, w.size(2), ptr_of<float>(xc), tokens, x.size(1),
+                                           ptr_of<int32_t>(ic), top_k, out_of<float>(y));
+        });
         return wrap(y);
     });
 }
@@ -409,9 +447,14 @@ PyObject *gather_qmm(PyObject *, Args a, Py_ssize_t na) {
         const size_t need = lisa_cuda_gather_qmm_workspace_bytes(rows, experts);
         if (!ws.defined() && need) ws = empty({static_cast<int64_t>(need)}, at::kByte, x);
         const at::Tensor ids = !rhs.defined() ? rhs : whole(rhs.scalar_type() == at::kInt ? rhs : rhs.to(at::kInt));
-        check(lisa_cuda_gather_qmm(stream, ptr(xc), rows, k, ptr_of<uint32_t>(w), ptr(s), ptr(b), ptr_of<int32_t>(lhs), ptr_of<int32_t>(ids),
-                                   experts, n, truth(a[6]), static_cast<int>(integer(a[7])), static_cast<int>(integer(a[8])), truth(a[9]),
-                                   dtype_code(xc), out_ptr(y), out_ptr(ws), ws.defined() ? static_cast<size_t>(ws.numel()) : 0));
+        const int transpose = truth(a[6]);
+        const int sorted = truth(a[9]);
+        const int gs = static_cast<int>(integer(a[7]));
+        const int bits = static_cast<int>(integer(a[8]));
+        enqueue([&] {
+            return lisa_cuda_gather_qmm(stream, ptr(xc), rows, k, ptr_of<uint32_t>(w), ptr(s), ptr(b), ptr_of<int32_t>(lhs), ptr_of<int32_t>(ids),
+                                   experts, n, transpose, gs, bits, sorted, dtype_code(xc), out_ptr(y), out_ptr(ws), ws.defined() ? static_cast<size_t>(ws.numel()) : 0);
+        });
         return wrap(y);
     });
 }
@@ -437,9 +480,13 @@ PyObject *gather_qmm_siblings(PyObject *, Args a, Py_ssize_t na) {
         }
         const size_t need = lisa_cuda_gather_qmm_workspace_bytes(rows, experts);
         if (!ws.defined() && need) ws = empty({static_cast<int64_t>(need)}, at::kByte, x);
-        check(lisa_cuda_gather_qmm_siblings(stream, ptr(xc), rows, k, l.count, l.w, l.s, l.b, ptr_of<int32_t>(ids), experts, n, 1,
-                                            static_cast<int>(integer(a[3])), static_cast<int>(integer(a[4])), 1, dtype_code(xc), l.out, out_ptr(ws),
-                                            ws.defined() ? static_cast<size_t>(ws.numel()) : 0));
+        const int gs = static_cast<int>(integer(a[3]));
+        const int bits = static_cast<int>(integer(a[4]));
+        enqueue([&] {
+            return lisa_cuda_gather_qmm_siblings(stream, ptr(xc), rows, k, l.count, l.w, l.s, l.b, ptr_of<int32_t>(ids), experts, n, 1,
+                                            gs, bits, 1, dtype_code(xc), l.out, out_ptr(ws),
+                                            ws.defined() ? static_cast<size_t>(ws.numel()) : 0);
+        });
         return list_of(l.y, l.count);
     });
 }
@@ -475,9 +522,13 @@ PyObject *moe_block(PyObject *, Args a, Py_ssize_t na) {
         const int top_k = static_cast<int>(integer(a[13]));
         const size_t need = lisa_cuda_moe_block_workspace_bytes(tokens, experts, top_k, hidden, inter);
         const at::Tensor ws = empty({static_cast<int64_t>(need)}, at::kByte, x), out = empty({tokens, hidden}, x);
-        check(lisa_cuda_moe_block(c10::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr_of<float>(logits), tokens, experts, top_k, hidden, inter, l.w[0], l.s[0], l.b[0],
+        const int64_t decode_slots = integer(a[14]);
+        const lisa_stream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+        enqueue([&] {
+            return lisa_cuda_moe_block(stream, ptr(xc), ptr_of<float>(logits), tokens, experts, top_k, hidden, inter, l.w[0], l.s[0], l.b[0],
                                   l.w[1], l.s[1], l.b[1], l.w[2], l.s[2], l.b[2], static_cast<int>(gs), static_cast<int>(bits),
-                                  dtype_code(xc), integer(a[14]), out_ptr(out), out_ptr(ws), need));
+                                  dtype_code(xc), decode_slots, out_ptr(out), out_ptr(ws), need);
+        });
         return wrap(out);
     });
 }

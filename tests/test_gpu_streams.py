@@ -75,3 +75,34 @@ def test_outputs_belong_to_the_current_stream(cuda):
     address = y.data_ptr()
     del y
     assert torch.empty((1, 128), dtype=torch.bfloat16, device=cuda).data_ptr() == address
+
+
+def test_a_launch_that_waits_for_its_stream_lets_other_threads_run(cuda):
+    """A stream's queue takes some thousand launches; the next one waits for the GPU.  It waits without the interpreter's lock."""
+    import threading
+    import time
+
+    rng = np.random.default_rng(3)
+    lin = _affine(cuda, rng, 128, 256)
+    x = dev_bf16(util.activations(rng, 1, 256), cuda)
+    out = ops.quantized_matmul(x, *lin)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(40 * SLEEP)  # about a second
+
+    def fill():
+        for _ in range(6000):
+            ops.quantized_matmul(x, *lin, out=out, stream=side)
+
+    worker, gap, last = threading.Thread(target=fill), 0.0, time.perf_counter()
+    worker.start()
+    start = last
+    while worker.is_alive():
+        now = time.perf_counter()
+        gap, last = max(gap, now - last), now
+        time.sleep(0)
+    side.synchronize()
+    took = time.perf_counter() - start
+    assert took > 0.4, "the queue took everything: the test shows nothing"
+    assert gap < 0.25, f"the other thread stood for {gap:.2f} s of {took:.2f}"
