@@ -3,7 +3,7 @@
 //   gate|up   act[slot, :] = swiglu(bf16(x . Wg[e]^T), bf16(x . Wu[e]^T))                  CTA = rows of one slot
 //   down      out[t, :] = bf16(fold_j f32(bf16(act[t, j] . Wd[e_j]^T)) * w[t, j])          CTA = rows of one token
 // What moe_gate_up_act and moe_down_combine compute (moe_decode.cu, with the reference's files), with their rounding points and
-// their fold.
+// their fold; like them it takes the activations as they are (four bytes each, see dp_core.cuh).
 //
 // At one token the block is latency, not bytes (21 MB of eight experts are 3.3 us at the copy rate; router, gate|up and down took
 // 36 us one after another).  Both launches are dependent ones: gate|up converts x while the router runs and waits for nothing
@@ -21,7 +21,7 @@ namespace lisa {
 
 namespace {
 
-constexpr int kMdThreads = 512, kMdWarps = kMdThreads / 32, kMdMaxTopK = 32;
+constexpr int kMdThreads = 512, kMdWarps = kMdThreads / 32, kMdMaxTopK = 32, kMdPlanes = 4;
 
 struct MoeDpParams {
     const int32_t *idx;   // [tokens, top_k] expert ids and weights of the router
@@ -39,7 +39,7 @@ struct MoeDpParams {
 
 template <int BITS, bool G32, bool DOWN>
 __global__ void __launch_bounds__(kMdThreads, 2) moe_dp_kernel(const MoeDpParams p) {
-    using S = DpShape<BITS>;
+    using S = DpShape<BITS, kMdPlanes>;
     using Take = DpTake<BITS, G32>;
     constexpr int XV = S::kXWords / 4, SUB = G32 ? 2 : 1, CB = S::kWords * 4, WSLOT = Take::kWSlot, SLOT = Take::kSlot, DEPTH = BITS == 2 ? 4 : 2;
     constexpr int MATS = DOWN ? 1 : 2;
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kMdThreads, 2) moe_dp_kernel(const MoeDpParams
         for (int i = tid; i < xrows * nv_pad; i += kMdThreads) {
             const int r = DOWN ? i / nv_pad : 0, v = i - r * nv_pad;
             const uint4 *src = reinterpret_cast<const uint4 *>(xr + static_cast<size_t>(r) * p.k);
-            dp_convert<BITS, G32>(xs + static_cast<size_t>(r) * p.steps * XV * 8, xf + static_cast<size_t>(r) * p.steps * 8 * (1 + SUB), v,
+            dp_convert<BITS, G32, kMdPlanes>(xs + static_cast<size_t>(r) * p.steps * XV * 8, xf + static_cast<size_t>(r) * p.steps * 8 * (1 + SUB), v,
                                   v < nv ? (DOWN ? __ldcg(src + v) : __ldg(src + v)) : make_uint4(0, 0, 0, 0));
         }
     };
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kMdThreads, 2) moe_dp_kernel(const MoeDpParams
             fetch();
             at += SLOT;
             if (at == ring_end) at = ring;
-            dp_chunk<BITS, G32>(w, sc, bi, xp, fp, mask, take.flip, acc0, acc1);
+            dp_chunk<BITS, G32, kMdPlanes>(w, sc, bi, xp, fp, mask, take.flip, acc0, acc1);
         }
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -269,7 +269,7 @@ bool md_plan(int64_t zs, int64_t n, int64_t k, int streams, int xrows, int group
         }
     }
     const int sub = group_size == 32 ? 2 : 1;
-    const int64_t xs = static_cast<int64_t>(xrows) * p.steps * 8 * 128, xf = static_cast<int64_t>(xrows) * p.steps * 8 * 4 * (1 + sub);
+    const int64_t xs = static_cast<int64_t>(xrows) * p.steps * 8 * 64 * kMdPlanes, xf = static_cast<int64_t>(xrows) * p.steps * 8 * 4 * (1 + sub);
     if (xs > (1 << 20)) return false;
     p.xf_at = static_cast<int>(xs);
     p.ring_at = static_cast<int>((xs + xf + 127) & ~127);

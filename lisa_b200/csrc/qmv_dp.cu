@@ -6,7 +6,8 @@
 // quantized.metal:762-1088) with the factorisation of the reference's qdot (quantized.metal:196-295) and the same
 // integer grid for the activations: with E the exponent of the largest magnitude of a chunk of x, x * 2^(13-E) is
 // rounded to an integer below 2^14 and split into two signed bytes; products and sums are exact in s32, scale and bias
-// are applied per chunk in f32.
+// are applied per chunk in f32.  That grid is what the operator promises for 2- and 4-bit codes with group size 64; 8-bit codes and group sizes
+// 32 and 128, whose other kernels take the activations as they are, use four bytes, 2^(29-E) (see dp_core.cuh).
 //
 // What bounds a decode launch is not the stream of weights (a 14 MB matrix is 95 KB per SM) but the chain in front of
 // and behind it: launch, activations, conversion, reduction.  So the kernel keeps that chain short:
@@ -60,11 +61,11 @@ struct DpParams {
     uint16_t *nsum, *nnorm;
 };
 
-// MT rows of x; DEPTH slots in a warp's ring
-template <int BITS, int FUSE, int MT, bool G32, int DEPTH>
+// MT rows of x; DEPTH slots in a warp's ring; PLANES bytes of an activation
+template <int BITS, int FUSE, int MT, bool G32, int DEPTH, int PLANES>
 __global__ void __launch_bounds__(kDpThreads, 2) qmv_dp_kernel(const DpParams p) {
-    using S = DpShape<BITS>;
-    constexpr int XV = S::kXWords / 4;  // 16-byte vectors of activation words per chunk: 8 / 8 / 4
+    using S = DpShape<BITS, PLANES>;
+    constexpr int XV = S::kXWords / 4;  // 16-byte vectors of activation words per chunk: 8 / 8 / 4 of two planes
     constexpr int SUB = G32 ? 2 : 1;    // scale groups of a chunk (group size 32 under 64 codes: two)
     constexpr int CB = S::kWords * 4;   // bytes of a chunk: 16 (2-bit) / 32
     constexpr int WSLOT = 64 * CB;      // packed bytes of a ring slot: eight rows x eight chunks
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(kDpThreads, 2) qmv_dp_kernel(const DpParams p)
                         if (p.nnorm) reinterpret_cast<uint4 *>(p.nnorm + static_cast<size_t>(t) * p.k)[i] = v;
                     }
                 }
-                dp_convert<BITS, G32>(xs_t, xf_t, i, v);
+                dp_convert<BITS, G32, PLANES>(xs_t, xf_t, i, v);
             };
             // (whole warps: nv_pad is a multiple of 32)
 #pragma unroll
@@ -264,10 +265,10 @@ __global__ void __launch_bounds__(kDpThreads, 2) qmv_dp_kernel(const DpParams p)
                 uint4 v0 = i0 < nv ? __ldg(reinterpret_cast<const uint4 *>(xr) + i0) : make_uint4(0, 0, 0, 0);
                 uint4 v1 = i1 < nv ? __ldg(reinterpret_cast<const uint4 *>(xr) + i1) : make_uint4(0, 0, 0, 0);
                 if (i0 < nv) v0 = vec(i0, v0);
-                dp_convert<BITS, G32>(xs_t, xf_t, i0, v0);
+                dp_convert<BITS, G32, PLANES>(xs_t, xf_t, i0, v0);
                 if (i1 < nv_pad) {
                     if (i1 < nv) v1 = vec(i1, v1);
-                    dp_convert<BITS, G32>(xs_t, xf_t, i1, v1);
+                    dp_convert<BITS, G32, PLANES>(xs_t, xf_t, i1, v1);
                 }
             }
         }
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(kDpThreads, 2) qmv_dp_kernel(const DpParams p)
 #pragma unroll
             for (int t = 0; t < MT; ++t) {
                 const uint32_t xt = xp + t * p.steps * (XV * 128), ft = fp + t * p.steps * (32 + 32 * SUB);
-                dp_chunk<BITS, G32>(w, sc, bi, xt, ft, mask, take.flip, acc[0][t], acc[1][t]);
+                dp_chunk<BITS, G32, PLANES>(w, sc, bi, xt, ft, mask, take.flip, acc[0][t], acc[1][t]);
             }
         }
         // the task's sums over its eight lanes, to their place in the order of k
@@ -342,6 +343,9 @@ __global__ void __launch_bounds__(kDpThreads, 2) qmv_dp_kernel(const DpParams p)
 struct DpPlan {
     int smem, grid, depth;
 };
+
+// Bytes of an activation (see the head of the file).
+constexpr int dp_planes(int group_size, int bits) { return bits == 8 || group_size != 64 ? 4 : 2; }
 
 // Cut of k into tasks and shared memory, from n (all the linears of the launch) and k only.
 bool dp_make_plan(int64_t octets, int64_t k, int group_size, int bits, int mt, DpParams &p, DpPlan &pl) {
@@ -380,18 +384,20 @@ bool dp_make_plan(int64_t octets, int64_t k, int group_size, int bits, int mt, D
         p.tail_bytes = p.row_bytes - (p.steps - 1) * 8 * (bits == 2 ? 16 : 32);
         p.tail_words = p.groups / 2 - (p.steps - 1) * p.scale_words;
     }
-    const size_t fixed = static_cast<size_t>(mt) * p.steps * 8 * (codes * 2 + 4 * (1 + sub)) + static_cast<size_t>(per) * 8 * p.parts * mt * 4;
+    const size_t fixed = static_cast<size_t>(mt) * p.steps * 8 * (codes * dp_planes(group_size, bits) + 4 * (1 + sub)) + static_cast<size_t>(per) * 8 * p.parts * mt * 4;
     p.ring_at = static_cast<int>((fixed + 127) & ~static_cast<size_t>(127));
     const int slot = 64 * (bits == 2 ? 16 : 32) + 256 * sub;
     const int full = bits == 2 ? 4 : 2;
-    for (int depth : {full, full / 2}) {
-        const size_t bytes = p.ring_at + static_cast<size_t>(kDpWarps) * depth * slot;
-        if (fixed < (1u << 20) && bytes <= static_cast<size_t>(max_smem_optin() / 2 - 2048)) {
-            pl.depth = depth;
-            pl.smem = static_cast<int>(bytes);
-            return true;
+    // half an SM, so that the next launch's weights come in beside this one; four planes of a long row: a whole one
+    for (int limit : {max_smem_optin() / 2 - 2048, dp_planes(group_size, bits) == 4 ? max_smem_optin() - 2048 : 0})
+        for (int depth : {full, full / 2}) {
+            const size_t bytes = p.ring_at + static_cast<size_t>(kDpWarps) * depth * slot;
+            if (fixed < (1u << 20) && bytes <= static_cast<size_t>(limit)) {
+                pl.depth = depth;
+                pl.smem = static_cast<int>(bytes);
+                return true;
+            }
         }
-    }
     return false;
 }
 
@@ -413,41 +419,36 @@ bool dp_plan(int64_t octets, int64_t k, int group_size, int bits, int mt, DpPara
     return e->ok;
 }
 
-template <int BITS, int FUSE, int MT, bool G32, int DEPTH>
+template <int BITS, int FUSE, int MT, bool G32, int DEPTH, int PLANES>
 int dp_launch_depth(cudaStream_t stream, const DpParams &p, const DpPlan &pl, unsigned flags) {
-    static std::atomic<uint64_t> ready{0};
-    const int rc = allow_smem(reinterpret_cast<const void *>(&qmv_dp_kernel<BITS, FUSE, MT, G32, DEPTH>), max_smem_optin() / 2, ready);
-    if (rc != LISA_OK) return rc;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(pl.grid);
-    cfg.blockDim = dim3(kDpThreads);
-    cfg.dynamicSmemBytes = pl.smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    if (flags & LISA_FLAG_PDL) {
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-    }
-    LISA_CUDA_TRY(cudaLaunchKernelEx(&cfg, qmv_dp_kernel<BITS, FUSE, MT, G32, DEPTH>, p));
+    LISA_TRY((allow_smem_of<qmv_dp_kernel<BITS, FUSE, MT, G32, DEPTH, PLANES>>()));
+    LISA_TRY(launch_kernel(stream, pl.grid, kDpThreads, pl.smem, flags, qmv_dp_kernel<BITS, FUSE, MT, G32, DEPTH, PLANES>, p));
     count_launch();
     return LISA_OK;
 }
 
-template <int BITS, int FUSE, int MT, bool G32>
+template <int BITS, int FUSE, int MT, bool G32, int PLANES>
 int dp_launch_one(cudaStream_t stream, const DpParams &p, const DpPlan &pl, unsigned flags) {
     constexpr int kFull = BITS == 2 ? 4 : 2;
-    return pl.depth == kFull ? dp_launch_depth<BITS, FUSE, MT, G32, kFull>(stream, p, pl, flags)
-                             : dp_launch_depth<BITS, FUSE, MT, G32, kFull / 2>(stream, p, pl, flags);
+    return pl.depth == kFull ? dp_launch_depth<BITS, FUSE, MT, G32, kFull, PLANES>(stream, p, pl, flags)
+                             : dp_launch_depth<BITS, FUSE, MT, G32, kFull / 2, PLANES>(stream, p, pl, flags);
 }
 
-template <int BITS, int FUSE>
-int dp_launch(cudaStream_t stream, const DpParams &p, const DpPlan &pl, int mt, bool g32, unsigned flags) {
-    if constexpr (BITS != 8 && FUSE == 0) {
-        if (g32) return mt == 2 ? dp_launch_one<BITS, 0, 2, true>(stream, p, pl, flags) : dp_launch_one<BITS, 0, 1, true>(stream, p, pl, flags);
+template <int BITS, int FUSE, bool G32, int PLANES>
+int dp_launch_rows(cudaStream_t stream, const DpParams &p, const DpPlan &pl, int mt, unsigned flags) {
+    return mt == 2 ? dp_launch_one<BITS, FUSE, 2, G32, PLANES>(stream, p, pl, flags) : dp_launch_one<BITS, FUSE, 1, G32, PLANES>(stream, p, pl, flags);
+}
+
+template <int BITS>
+int dp_launch(cudaStream_t stream, const DpParams &p, const DpPlan &pl, int mt, int fuse, int group_size, unsigned flags) {
+    if constexpr (BITS == 8) {
+        return dp_launch_rows<8, 0, false, 4>(stream, p, pl, mt, flags);
+    } else {
+        if (fuse == 1) return dp_launch_rows<BITS, 1, false, 2>(stream, p, pl, mt, flags);
+        if (fuse == 2) return dp_launch_rows<BITS, 2, false, 2>(stream, p, pl, mt, flags);
+        if (group_size == 64) return dp_launch_rows<BITS, 0, false, 2>(stream, p, pl, mt, flags);
+        return group_size == 32 ? dp_launch_rows<BITS, 0, true, 4>(stream, p, pl, mt, flags) : dp_launch_rows<BITS, 0, false, 4>(stream, p, pl, mt, flags);
     }
-    return mt == 2 ? dp_launch_one<BITS, FUSE, 2, false>(stream, p, pl, flags) : dp_launch_one<BITS, FUSE, 1, false>(stream, p, pl, flags);
 }
 
 int64_t dp_octets(int count, const int64_t *n) {
@@ -500,11 +501,9 @@ int qmv_dp(cudaStream_t stream, const void *x, int64_t m, int64_t k, int count, 
             p.nsum = norm->sum ? reinterpret_cast<uint16_t *>(norm->sum) + done * k : nullptr;
             p.nnorm = norm->normed ? reinterpret_cast<uint16_t *>(norm->normed) + done * k : nullptr;
         }
-        const bool g32 = group_size == 32;
-        int rc;
-        if (bits == 4) rc = fuse == 1 ? dp_launch<4, 1>(stream, p, pl, mt, false, flags) : fuse == 2 ? dp_launch<4, 2>(stream, p, pl, mt, false, flags) : dp_launch<4, 0>(stream, p, pl, mt, g32, flags);
-        else if (bits == 2) rc = fuse == 1 ? dp_launch<2, 1>(stream, p, pl, mt, false, flags) : fuse == 2 ? dp_launch<2, 2>(stream, p, pl, mt, false, flags) : dp_launch<2, 0>(stream, p, pl, mt, g32, flags);
-        else rc = dp_launch<8, 0>(stream, p, pl, mt, false, flags);
+        const int rc = bits == 4   ? dp_launch<4>(stream, p, pl, mt, fuse, group_size, flags)
+                       : bits == 2 ? dp_launch<2>(stream, p, pl, mt, fuse, group_size, flags)
+                                   : dp_launch<8>(stream, p, pl, mt, fuse, group_size, flags);
         if (rc != LISA_OK) return rc;
         done += mt;
     }
