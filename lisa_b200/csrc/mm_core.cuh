@@ -73,10 +73,10 @@ __device__ __forceinline__ void mm_fragment(const uint32_t (&e)[8], uint32_t fra
         sum += __shfl_xor_sync(0xffffffffu, sum, off);
         amax = __vmaxu2(amax, __shfl_xor_sync(0xffffffffu, amax, off));
     }
-    // E: biased exponent of the group's largest magnitude.  Groups below 2^-113 count as zero; an infinity or NaN makes the
-    // factor NaN.
-    const uint32_t ex = max(amax & 0xffffu, amax >> 16) >> 7;
-    const bool live = ex >= 14u && ex < 255u;
+    // E: biased exponent of the group's largest magnitude, at least the one whose inverse is a float (smaller groups keep that grid).  An
+    // infinity or NaN makes the factor NaN.
+    const uint32_t ex0 = max(amax & 0xffffu, amax >> 16) >> 7, ex = max(ex0, 14u);
+    const bool live = ex0 < 255u;
     const float up = live ? __uint_as_float((268u - ex) << 23) : 0.f;  // 2^(14 - (E - 127))
     auto lo = [&](int i) { return __uint_as_float(e[i] << 16); };
     auto hi = [&](int i) { return __uint_as_float(e[i] & 0xffff0000u); };
@@ -110,7 +110,7 @@ __device__ __forceinline__ void mm_fragment(const uint32_t (&e)[8], uint32_t fra
         if (cc == 0) {
             const uint32_t so = sums + gl * SUMS + (t >> 1) * 16 + (t & 1) * 4;
             // 2^((E - 127) - 14 + 24), less the 2^16 that the scale takes (each stays in range)
-            const float factor = live ? __uint_as_float((ex - 6u) << 23) : (ex == 255u ? __uint_as_float(0x7fc00000u) : 0.f);
+            const float factor = __uint_as_float(live ? (ex - 6u) << 23 : 0x7fc00000u);
             asm volatile("st.shared.f32 [%0], %1;" ::"r"(so), "f"(factor) : "memory");
             asm volatile("st.shared.f32 [%0], %1;" ::"r"(so + 8), "f"(sum) : "memory");
         }

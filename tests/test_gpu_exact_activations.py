@@ -45,6 +45,22 @@ def test_heavy_tails(cuda, bits, gs, n, k, m, ratio):
     assert np.all(np.abs(O.bf16_to_f32(host_bf16_bits(y)) - truth) <= 2.0 ** -8 * np.abs(truth) + 2.0 ** -16 * terms)
 
 
+@pytest.mark.parametrize("scale", [2.0 ** -100, 2.0 ** -118])
+@pytest.mark.parametrize("bits,gs,m", [(8, 64, 1), (8, 64, 4), (4, 128, 2), (4, 128, 8), (4, 32, 1), (2, 128, 3)])
+def test_small_activations_are_not_zeros(cuda, bits, gs, m, scale):
+    """Groups of very small elements: the kernels' grids follow them down to the range of a float."""
+    rng = np.random.default_rng(bits + gs + m)
+    n, k = 64, 512
+    w, s, b = util.affine_weights(rng, n, k, bits, gs)
+    x = O.f32_to_bf16((O.bf16_to_f32(util.activations(rng, m, k)) * np.float32(scale)).astype(np.float32))
+    y = ops.quantized_matmul(dev_bf16(x, cuda), dev_u32(w, cuda), dev_bf16(s, cuda), dev_bf16(b, cuda), True, gs, bits)
+    truth = O.bf16_to_f32(x).astype(np.float64) @ O.affine_dequantize(w, s, b, gs, bits, out_f32=True).astype(np.float64).T
+    err = np.abs(O.bf16_to_f32(host_bf16_bits(y)).astype(np.float64) - truth)
+    # (2^-122 is the grid of four bytes at its lower end, 2^-133 the smallest bf16)
+    assert np.all(err <= 2.0 ** -8 * np.abs(truth) + 2.0 ** -12 * np.sqrt(np.mean(truth * truth)) + 2.0 ** -117)
+    assert np.linalg.norm(err) <= (2.0 ** -7 if scale > 2.0 ** -110 else 0.05) * np.linalg.norm(truth)
+
+
 @pytest.mark.parametrize("gs", [32, 64, 128])
 @pytest.mark.parametrize("bits", [4, 2])
 @pytest.mark.parametrize("tokens", [1, 3, 9])
