@@ -552,6 +552,12 @@ static int gguf_geometry(const char *op, int format, int64_t rows, int64_t row_b
     return LISA_OK;
 }
 
+// Calls whose activations are on the documented grid (2^-21 of a sub-block's largest): one token, or up to 256 slots of the expert form, over
+// 16-byte aligned rows of whole stages -- what the tensor-memory kernel takes.  All others see f32 activations.
+static bool gguf_grid_call(int format, const uint8_t *w, int64_t zs, int64_t rows, int64_t row_bytes, bool experts) {
+    return aligned16(w) && row_bytes % (format == LISA_GGUF_Q2_K ? 336 : 144) == 0 && zs <= (experts ? 256 : 1) && rows <= (1 << 24);
+}
+
 int lisa_cuda_gguf_packed_matvec(lisa_stream_t stream, int format, const uint8_t *w, int64_t rows, int64_t row_bytes,
                                  const float *x, int64_t tokens, float *y) {
     int block = 0;
@@ -563,10 +569,10 @@ int lisa_cuda_gguf_packed_matvec(lisa_stream_t stream, int format, const uint8_t
     if (!aligned16(x) || (reinterpret_cast<uintptr_t>(y) & 3u) != 0)
         return fail(LISA_ERR_MISALIGNED, "packed_matvec: x must be 16-byte and y 4-byte aligned");
     // one token: the byte form (17.8 against 22.6 us on Q4_K 18432 x 7168); more: one pass over the weights for up to eight
-    if (tokens > 1 && gguf_mm_supported(format, w, tokens, rows, row_bytes))
+    if (gguf_grid_call(format, w, tokens, rows, row_bytes, false) && gguf_dp_supported(format, w, tokens, rows, row_bytes, false, false))
+        return gguf_dp(static_cast<cudaStream_t>(stream), format, w, 1, rows, row_bytes, x, tokens, 1, nullptr, 1, y, false);
+    if (gguf_mm_supported(format, w, tokens, rows, row_bytes))
         return gguf_mm(static_cast<cudaStream_t>(stream), format, w, rows, row_bytes, x, tokens, y);
-    if (gguf_dp_supported(format, w, tokens, rows, row_bytes, false))
-        return gguf_dp(static_cast<cudaStream_t>(stream), format, w, 1, rows, row_bytes, x, tokens, 1, nullptr, 1, y);
     // one or two tokens of a Q4_K matrix: the tensor-memory kernel (exact on dyadic inputs like the warp-per-row one)
     if (aligned16(w) && row_bytes % 16 == 0 && qmv_tc_gguf_supported(format, tokens, rows, row_bytes))
         return qmv_tc_gguf(static_cast<cudaStream_t>(stream), format, w, rows, row_bytes, x, tokens, y);
@@ -633,8 +639,9 @@ int lisa_cuda_gguf_expert_matvec(lisa_stream_t stream, int format, const uint8_t
     if ((reinterpret_cast<uintptr_t>(w) & 1u) != 0) return fail(LISA_ERR_MISALIGNED, "expert_matvec: weights must be 2-byte aligned");
     if (!aligned16(x) || (reinterpret_cast<uintptr_t>(y) & 3u) != 0 || (reinterpret_cast<uintptr_t>(ids) & 3u) != 0)
         return fail(LISA_ERR_MISALIGNED, "expert_matvec: x must be 16-byte, y and ids 4-byte aligned");
-    if (gguf_dp_supported(format, w, tokens * top_k, rows, row_bytes, true))
-        return gguf_dp(static_cast<cudaStream_t>(stream), format, w, experts, rows, row_bytes, x, tokens * top_k, slots, ids, top_k, y);
+    const bool exact = !gguf_grid_call(format, w, tokens * top_k, rows, row_bytes, true);
+    if (gguf_dp_supported(format, w, tokens * top_k, rows, row_bytes, true, exact))
+        return gguf_dp(static_cast<cudaStream_t>(stream), format, w, experts, rows, row_bytes, x, tokens * top_k, slots, ids, top_k, y, exact);
     // decode-sized id tables: every slot as a one-token launch tile of the tensor-memory kernel (exact on dyadic
     // inputs like the warp-per-row kernel; ids outside the table store zeros and touch no weights there too)
     if (aligned16(w) && row_bytes % 16 == 0 && qmv_tc_gguf_expert_supported(format, tokens * top_k, experts, rows, row_bytes))

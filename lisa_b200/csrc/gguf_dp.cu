@@ -5,9 +5,11 @@
 //
 // The structure is that of qmv_dp.cu: a warp walks tasks (eight rows, a run of steps) through a ring of asynchronous copies
 // of contiguous pieces of the rows -- block headers and codes as they lie in memory -- and multiplies bytes with dp4a.
-// An activation is three signed bytes on an integer grid of its sub-block (32 elements, Q2_K: 16): with E the exponent of
-// the sub-block's largest magnitude x_int = rn(x * 2^(21-E)) = 65536 p0 + 256 p1 + p2, 22 bits, exact on dyadic inputs; sums are
-// exact in s32 and meet scale and min of the sub-block in f32.
+// An activation is three or four signed bytes on an integer grid of its sub-block (32 elements, Q2_K: 16): with E the exponent of
+// the sub-block's largest magnitude x_int = rn(x * 2^(21-E)) or rn(x * 2^(29-E)), exact on dyadic inputs; sums are
+// exact in s32 and meet scale and min of the sub-block in f32.  Three bytes are the grid of the tensor-memory kernel, for the calls which that
+// one takes (gguf_grid_call in api.cu); all others are promised f32 activations, of which four bytes lose less than
+// f32 sums do: 2048 x 2304 of Q2_K, Gaussian activations, relative error 0.7e-7, the warp-per-row kernel 1.0e-7, three bytes 2.8e-7.
 //
 // Why not the tensor-memory kernel: its Q2_K stages took 42 KB, one CTA per SM and two stages, and both formats paid its
 // hand-overs per pair of k-blocks.  This form is bound by its instruction stream, about 0.06 warp instructions per code
@@ -71,23 +73,31 @@ __device__ __forceinline__ void gd_half2(uint32_t v, float &lo, float &hi) {
     asm("{ .reg .b16 l, h; mov.b32 {l, h}, %2; cvt.f32.f16 %0, l; cvt.f32.f16 %1, h; }" : "=f"(lo), "=f"(hi) : "r"(v));
 }
 
+// The sum that the planes' sums (the highest first, below 2^22 each) stand for.
+template <int PLANES>
+__device__ __forceinline__ float gd_value(const int (&c)[PLANES]) {
+    if constexpr (PLANES == 3) return fmaf(static_cast<float>(c[0]), 65536.f, static_cast<float>(c[1] * 256 + c[2]));
+    else return fmaf(static_cast<float>(c[0] * 256 + c[1]), 65536.f, static_cast<float>(c[2] * 256 + c[3]));
+}
+
 // FMT 4: Q4_K, a step is two blocks of a row, a lane's chunk 64 elements (32 code bytes, two sub-blocks); FMT 2: Q2_K, a step is
 // four blocks, a chunk 128 elements (32 code bytes, eight sub-blocks).  PIECE: bytes of a copy (16; 4 for Q2_K rows that are
 // not whole 16-byte pieces).
-template <int FMT>
+template <int FMT, int PLANES = 3>
 struct GdShape {
     static constexpr int kBlock = FMT == 4 ? 144 : 84;
     static constexpr int kBlocks = FMT == 4 ? 2 : 4;       // of a step
     static constexpr int kRow = kBlock * kBlocks;          // bytes of a row and step: 288 / 336
     static constexpr int kPitch = FMT == 4 ? 320 : 352;    // of the rows in a slot: room for 16 bytes of offset, whole sectors
     static constexpr int kElems = FMT == 4 ? 64 : 128;     // of a chunk
-    static constexpr int kXV = FMT == 4 ? 12 : 24;         // 16-byte vectors of activation words of a chunk
+    static constexpr int kXV = PLANES * (FMT == 4 ? 4 : 8);  // 16-byte vectors of activation words of a chunk
     static constexpr int kSubs = FMT == 4 ? 2 : 8;         // sub-blocks of a chunk
+    static constexpr int kGrid = PLANES == 3 ? 21 : 29;
 };
 
-template <int FMT, int PIECE>
+template <int FMT, int PIECE, int PLANES>
 __global__ void __launch_bounds__(kGdThreads, 1) gguf_dp_kernel(const GdParams p) {
-    using S = GdShape<FMT>;
+    using S = GdShape<FMT, PLANES>;
     constexpr int SLOT = 8 * S::kPitch, PPR = S::kRow / PIECE;  // pieces per row
     constexpr int COPIES = (8 * PPR + 31) / 32;
     extern __shared__ __align__(128) uint8_t gd_smem[];
@@ -207,40 +217,49 @@ __global__ void __launch_bounds__(kGdThreads, 1) gguf_dp_kernel(const GdParams p
                 amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, off));
                 sum += __shfl_xor_sync(0xffffffffu, sum, off);
             }
-            // E: biased exponent of the sub-block's largest magnitude; below 2^-105 the sub-block counts as zero, an infinity or
-            // NaN makes its factor NaN
-            const uint32_t e = amax >> 23;
-            const bool live = e >= 22u && e < 255u;
-            const float up = live ? __uint_as_float((275u - e) << 23) : 0.f;  // 2^(21 - (E - 127))
-            uint32_t b2[8], b1[8], b0[8];  // the three bytes in the low, second and third byte of a word each
+            // E: biased exponent of the sub-block's largest magnitude, at least the one whose factor is a float (smaller sub-blocks keep
+            // that grid); an infinity or NaN makes its factor NaN
+            const uint32_t e0 = amax >> 23, e = max(e0, S::kGrid + 7u);
+            const bool live = e0 < 255u;
+            const float up = live ? __uint_as_float((254u + S::kGrid - e) << 23) : 0.f;  // 2^(kGrid - (E - 127))
+            uint32_t digit[PLANES][8];  // the signed bytes of x_int, the highest first, each with its carry: digit q in byte PLANES - 1 - q of its word
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const int xi = live ? __float2int_rn(f[j] * up) : 0;  // |xi| < 2^22
-                b2[j] = static_cast<uint32_t>(xi);                    // byte 0
-                b1[j] = static_cast<uint32_t>(xi + 128);              // byte 1: (xi + 128) >> 8, and the carry into byte 2 below
-                b0[j] = static_cast<uint32_t>(xi + 128 + 32768);      // byte 2: (((xi + 128) >> 8) + 128) >> 8
+                const uint32_t xi = static_cast<uint32_t>(live ? __float2int_rn(f[j] * up) : 0);  // below 2^(kGrid + 1)
+                digit[PLANES - 1][j] = xi;
+                digit[PLANES - 2][j] = xi + 128u;
+                digit[PLANES - 3][j] = xi + 32896u;
+                if constexpr (PLANES == 4) digit[0][j] = xi + 8421504u;
             }
-            auto pack = [](const uint32_t *b, int at, uint32_t sel) { return __byte_perm(__byte_perm(b[at], b[at + 1], sel), __byte_perm(b[at + 2], b[at + 3], sel), 0x5410); };
+            auto pack = [&](int q, int at) {
+                constexpr uint32_t kSel[4] = {0x0040, 0x0051, 0x0062, 0x0073};
+                const uint32_t sel = kSel[PLANES - 1 - q];
+                return __byte_perm(__byte_perm(digit[q][at], digit[q][at + 1], sel), __byte_perm(digit[q][at + 2], digit[q][at + 3], sel), 0x5410);
+            };
             const int chunk = i / (S::kElems / 8), j = i - chunk * (S::kElems / 8);
             const uint32_t to = xs + (chunk >> 3) * (S::kXV * 128) + (chunk & 7) * 16;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const uint32_t pl[3] = {pack(b0, 4 * h, 0x0062), pack(b1, 4 * h, 0x0051), pack(b2, 4 * h, 0x0040)};
+                const int v_ = (j & 3) * 2 + h;  // packed word of these four elements; j / 4: the half or field of it
+                if constexpr (PLANES == 4) {
+                    // a vector per packed word and half (Q4_K) or field (Q2_K)
+                    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(to + ((FMT == 4 ? 2 : 4) * v_ + (j >> 2)) * 128), "r"(pack(0, 4 * h)),
+                                 "r"(pack(1, 4 * h)), "r"(pack(2, 4 * h)), "r"(pack(3, 4 * h)) : "memory");
+                } else {
 #pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    // Q4_K: word v of half s (low / high nibbles) at 6 (v & 1) + 3 s + q of its pair; Q2_K: word v of field f at 3 f + q
-                    const int v_ = FMT == 4 ? (j & 3) * 2 + h : (j & 3) * 2 + h;
-                    const int idx = FMT == 4 ? 6 * (v_ & 1) + 3 * (j >> 2) + q : 3 * (j >> 2) + q;
-                    const int vec = FMT == 4 ? 3 * (v_ >> 1) + (idx >> 2) : 3 * v_ + (idx >> 2);
-                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(to + vec * 128 + (idx & 3) * 4), "r"(pl[q]) : "memory");
+                    for (int q = 0; q < 3; ++q) {
+                        // Q4_K: word v of half s (low / high nibbles) at 6 (v & 1) + 3 s + q of its pair; Q2_K: word v of field f at 3 f + q
+                        const int idx = FMT == 4 ? 6 * (v_ & 1) + 3 * (j >> 2) + q : 3 * (j >> 2) + q;
+                        const int vec = FMT == 4 ? 3 * (v_ >> 1) + (idx >> 2) : 3 * v_ + (idx >> 2);
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(to + vec * 128 + (idx & 3) * 4), "r"(pack(q, 4 * h)) : "memory");
+                    }
                 }
             }
             if (j % IPS == 0) {
                 // Q4_K: sub-block j / 4 (its high nibbles carry 16); Q2_K: field f = j / 4 (it carries 4^f), half (j & 3) / 2
                 const int sb = FMT == 4 ? j >> 2 : (j >> 2) * 2 + ((j & 3) >> 1);
                 const uint32_t place = FMT == 4 ? 4u * (j >> 2) : 2u * (j >> 2);
-                const float factor = live ? __uint_as_float((e - 21u) << 23) * __uint_as_float((127u - place) << 23)
-                                          : (e == 255u ? __uint_as_float(0x7fc00000u) : 0.f);
+                const float factor = __uint_as_float(live ? (e - S::kGrid - place) << 23 : 0x7fc00000u);
                 asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xf + (chunk * S::kSubs + sb) * 8), "f"(factor), "f"(sum) : "memory");
             }
         }
@@ -275,11 +294,26 @@ __global__ void __launch_bounds__(kGdThreads, 1) gguf_dp_kernel(const GdParams p
                     gd_lds128(blk + 16 + (sl & 3) * 32, cw[r]);
                     gd_lds128(blk + 32 + (sl & 3) * 32, cw[r] + 4);
                 }
-                int c[2][2][3];  // [row][low, high nibbles][plane]
+                int c[2][2][PLANES];  // [row][low, high nibbles][plane]
 #pragma unroll
                 for (int r = 0; r < 2; ++r)
 #pragma unroll
-                    for (int s = 0; s < 2; ++s) c[r][s][0] = c[r][s][1] = c[r][s][2] = 0;
+                    for (int s = 0; s < 2; ++s)
+#pragma unroll
+                        for (int q = 0; q < PLANES; ++q) c[r][s][q] = 0;
+                if constexpr (PLANES == 4) {
+#pragma unroll
+                    for (int v = 0; v < 8; ++v)
+#pragma unroll
+                        for (int s = 0; s < 2; ++s) {
+                            uint32_t xw[4];
+                            gd_lds128(xp + (2 * v + s) * 128, xw);
+#pragma unroll
+                            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                                for (int q = 0; q < 4; ++q) c[r][s][q] = gd_dp4a(cw[r][v] & mask[s], xw[q], c[r][s][q]);
+                        }
+                } else
 #pragma unroll
                 for (int vp = 0; vp < 4; ++vp) {
                     uint32_t xw[12];
@@ -312,7 +346,7 @@ __global__ void __launch_bounds__(kGdThreads, 1) gguf_dp_kernel(const GdParams p
                     float as = 0.f, am = 0.f;  // sums under the block's d and dmin
 #pragma unroll
                     for (int s = 0; s < 2; ++s) {
-                        const float val = fmaf(static_cast<float>(c[r][s][0]), 65536.f, static_cast<float>(c[r][s][1] * 256 + c[r][s][2]));
+                        const float val = gd_value<PLANES>(c[r][s]);
                         as = fmaf(static_cast<float>((sc2 >> (8 * s)) & 255u), val * fs[2 * s], as);
                         am = fmaf(static_cast<float>((mn2 >> (8 * s)) & 255u), fs[2 * s + 1], am);
                     }
@@ -332,13 +366,27 @@ __global__ void __launch_bounds__(kGdThreads, 1) gguf_dp_kernel(const GdParams p
                 }
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    int c[2][4][3];  // [row][field][plane] of a 16-element sub-block
+                    int c[2][4][PLANES];  // [row][field][plane] of a 16-element sub-block
 #pragma unroll
                     for (int r = 0; r < 2; ++r)
 #pragma unroll
-                        for (int f = 0; f < 4; ++f) c[r][f][0] = c[r][f][1] = c[r][f][2] = 0;
+                        for (int f = 0; f < 4; ++f)
+#pragma unroll
+                            for (int q = 0; q < PLANES; ++q) c[r][f][q] = 0;
 #pragma unroll
                     for (int v = 4 * half; v < 4 * half + 4; ++v) {
+                        if constexpr (PLANES == 4) {
+#pragma unroll
+                            for (int f = 0; f < 4; ++f) {
+                                uint32_t xw[4];
+                                gd_lds128(xp + (4 * v + f) * 128, xw);
+#pragma unroll
+                                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                                    for (int q = 0; q < 4; ++q) c[r][f][q] = gd_dp4a(cw[r][v] & mask[f], xw[q], c[r][f][q]);
+                            }
+                            continue;
+                        } else {
                         uint32_t xw[12];
 #pragma unroll
                         for (int u = 0; u < 3; ++u) gd_lds128(xp + (3 * v + u) * 128, xw + 4 * u);
@@ -350,6 +398,7 @@ __global__ void __launch_bounds__(kGdThreads, 1) gguf_dp_kernel(const GdParams p
 #pragma unroll
                                 for (int q = 0; q < 3; ++q) c[r][f][q] = gd_dp4a(wf, xw[3 * f + q], c[r][f][q]);
                             }
+                        }
                     }
 #pragma unroll
                     for (int f = 0; f < 4; ++f) {
@@ -358,7 +407,7 @@ __global__ void __launch_bounds__(kGdThreads, 1) gguf_dp_kernel(const GdParams p
 #pragma unroll
                         for (int r = 0; r < 2; ++r) {
                             const uint32_t byte = (sc[r][f >> 1] >> (16 * (f & 1) + 8 * half)) & 255u;  // scale byte 2 f + half
-                            const float val = fmaf(static_cast<float>(c[r][f][0]), 65536.f, static_cast<float>(c[r][f][1] * 256 + c[r][f][2]));
+                            const float val = gd_value<PLANES>(c[r][f]);
                             as[r] = fmaf(static_cast<float>(byte & 15u), val * factor, as[r]);
                             am[r] = fmaf(static_cast<float>(byte >> 4), sum, am[r]);
                         }
@@ -396,7 +445,7 @@ struct GdPlan {
     int smem, piece;
 };
 
-GdPlan gd_make_plan(int fmt, int64_t zs, int64_t rows, int64_t row_bytes) {
+GdPlan gd_make_plan(int fmt, int64_t zs, int64_t rows, int64_t row_bytes, bool exact) {
     GdPlan pl{};
     const int block = fmt == 4 ? 144 : 84, blocks = fmt == 4 ? 2 : 4;
     const int64_t nb = row_bytes / block;
@@ -425,7 +474,7 @@ GdPlan gd_make_plan(int fmt, int64_t zs, int64_t rows, int64_t row_bytes) {
             p.spt = spt;
         }
     }
-    const int xv = fmt == 4 ? 12 : 24, subs = fmt == 4 ? 2 : 8;
+    const int xv = (exact ? 4 : 3) * (fmt == 4 ? 4 : 8), subs = fmt == 4 ? 2 : 8;
     const int64_t fixed = static_cast<int64_t>(p.steps) * (xv * 128 + 8 * subs * 8);
     if (fixed > (1 << 20)) return pl;
     p.ring_at = static_cast<int>((fixed + 127) & ~127);
@@ -437,40 +486,40 @@ GdPlan gd_make_plan(int fmt, int64_t zs, int64_t rows, int64_t row_bytes) {
     return pl;
 }
 
-bool gd_plan(int fmt, int64_t zs, int64_t rows, int64_t row_bytes, GdPlan &out) {
+bool gd_plan(int fmt, int64_t zs, int64_t rows, int64_t row_bytes, bool exact, GdPlan &out) {
     static thread_local PlanTable<GdPlan> table;
     bool known;
-    GdPlan *e = table.find(zs, rows, (row_bytes << 12) | (static_cast<int64_t>(current_device()) << 4) | fmt, known);
-    if (!known) *e = gd_make_plan(fmt, zs, rows, row_bytes);
+    GdPlan *e = table.find(zs, rows, (row_bytes << 12) | (static_cast<int64_t>(current_device()) << 4) | (exact ? 8 : 0) | fmt, known);
+    if (!known) *e = gd_make_plan(fmt, zs, rows, row_bytes, exact);
     out = *e;
     return out.ok;
 }
 
-template <int FMT, int PIECE>
+template <int FMT, int PIECE, int PLANES>
 int gd_launch(cudaStream_t stream, const GdPlan &pl, int64_t zs) {
-    LISA_TRY((allow_smem_of<gguf_dp_kernel<FMT, PIECE>>()));
-    LISA_TRY(launch_kernel(stream, static_cast<unsigned>(zs * pl.p.ctas), kGdThreads, pl.smem, 0, gguf_dp_kernel<FMT, PIECE>, pl.p));
+    LISA_TRY((allow_smem_of<gguf_dp_kernel<FMT, PIECE, PLANES>>()));
+    LISA_TRY(launch_kernel(stream, static_cast<unsigned>(zs * pl.p.ctas), kGdThreads, pl.smem, 0, gguf_dp_kernel<FMT, PIECE, PLANES>, pl.p));
     count_launch();
     return LISA_OK;
 }
 
 }  // namespace
 
-// The formats and shapes the kernel takes: Q4_K and Q2_K, one to eight tokens, or up to 1024 (token, expert) slots; 16-byte
-// aligned packed rows (Q2_K: 4-byte aligned ones too).
-bool gguf_dp_supported(int format, const void *w, int64_t zs, int64_t rows, int64_t row_bytes, bool experts) {
+// The formats and shapes the kernel takes: Q4_K and Q2_K, one token, or up to 1024 (token, expert) slots; 16-byte
+// aligned packed rows (Q2_K: 4-byte aligned ones too).  `exact`: four bytes an activation instead of three.
+bool gguf_dp_supported(int format, const void *w, int64_t zs, int64_t rows, int64_t row_bytes, bool experts, bool exact) {
     if (format != LISA_GGUF_Q4_K && format != LISA_GGUF_Q2_K) return false;
-    if (zs < 1 || zs > (experts ? 1024 : 8)) return false;
+    if (zs < 1 || zs > (experts ? 1024 : 1)) return false;
     GdPlan pl;
-    if (!gd_plan(format == LISA_GGUF_Q4_K ? 4 : 2, zs, rows, row_bytes, pl)) return false;
+    if (!gd_plan(format == LISA_GGUF_Q4_K ? 4 : 2, zs, rows, row_bytes, exact, pl)) return false;
     return (reinterpret_cast<uintptr_t>(w) & static_cast<uintptr_t>(pl.piece - 1)) == 0;
 }
 
 int gguf_dp(cudaStream_t stream, int format, const uint8_t *w, int64_t experts, int64_t rows, int64_t row_bytes, const float *x, int64_t zs,
-            int64_t slots, const int32_t *ids, int64_t top_k, float *y) {
+            int64_t slots, const int32_t *ids, int64_t top_k, float *y, bool exact) {
     GdPlan pl;
     const bool q4 = format == LISA_GGUF_Q4_K;
-    if (!gd_plan(q4 ? 4 : 2, zs, rows, row_bytes, pl)) return fail(LISA_ERR_UNSUPPORTED, "gguf_dp: shape not supported");
+    if (!gd_plan(q4 ? 4 : 2, zs, rows, row_bytes, exact, pl)) return fail(LISA_ERR_UNSUPPORTED, "gguf_dp: shape not supported");
     pl.p.w = w;
     pl.p.x = x;
     pl.p.y = y;
@@ -478,8 +527,12 @@ int gguf_dp(cudaStream_t stream, int format, const uint8_t *w, int64_t experts, 
     pl.p.experts = static_cast<int>(experts);
     pl.p.slots = static_cast<int>(slots);
     pl.p.top_k = static_cast<int>(top_k);
-    if (q4) return gd_launch<4, 16>(stream, pl, zs);
-    return pl.piece == 16 ? gd_launch<2, 16>(stream, pl, zs) : gd_launch<2, 4>(stream, pl, zs);
+    if (exact) {
+        if (q4) return gd_launch<4, 16, 4>(stream, pl, zs);
+        return pl.piece == 16 ? gd_launch<2, 16, 4>(stream, pl, zs) : gd_launch<2, 4, 4>(stream, pl, zs);
+    }
+    if (q4) return gd_launch<4, 16, 3>(stream, pl, zs);
+    return pl.piece == 16 ? gd_launch<2, 16, 3>(stream, pl, zs) : gd_launch<2, 4, 3>(stream, pl, zs);
 }
 
 }  // namespace lisa

@@ -1,14 +1,19 @@
-// GGUF K-quant matvec for two tokens and more on mma.sync with f16 operands: f32 activations and output.
+// GGUF K-quant matvec on mma.sync, for two tokens and more (and for one where gguf_dp.cu's grid is not asked for), with f16 operands: f32 activations and output.
 //   y[z, r] = sum_k x[z, k] * W[e(z), r, k],  Q4_K and Q2_K blocks (crates/lisa-gguf/src/quant.rs:64-101)
 // (deepseek41::packed_matvec, crates/lisa-mlx/src/models/deepseek41.rs:93-283; its Metal kernels crates/lisa-mlx/src/shaders/deepseek41/iq.metal:1130-1363).
 //
-// Operands without loss: a masked code is a subnormal f16 (q * place * 2^-24 exactly), times its sub-block's integer scale (divided by
-// the place) one f16 multiplication, exact (at most ten bits); so all codes of a 256-element block meet one accumulator, and d, dmin
+// Operands without loss: a code in the mantissa of 1024 (one LOP3) goes through one f16 multiply-add with its sub-block's integer scale, divided by
+// the code's place in the byte: q * scale exactly (at most ten bits); so all codes of a 256-element block meet one scale, and d, dmin
 // follow per block in f32.  An f32 activation, normalised by a power of two per block, is the sum of three f16 (33 bits): three of
-// the MMA's columns per token.  The minima are one more MMA per block against the
-// sums of sixteen activations.
+// the MMA's columns per token.  The minima are one more MMA per block against the sums of sixteen activations.
 //
-// What bounds it: per code 5/8 (4/8 at 2 bits) of an operation of the half-rate pipe and half a packed multiplication, 0.055 warp
+// Sums: an MMA aligns its products and its accumulator to the largest of them by its exponent field and cuts what is below some 24 bits.  So
+// operands are normal numbers (with codes as subnormals, which the products' exponents do not tell from numbers near 2^-14, the sums of Q2_K
+// lost five bits), and an accumulator takes two MMAs, 32 products; everything else is added in f32.  Relative error (2-norm) on Gaussian
+// activations, Q4_K / Q2_K, 1208 x 1280, four tokens: 1.1e-7 / 0.8e-7 (one accumulator a block 2.9e-7 / 1.1e-7, the warp-per-row kernel
+// 1.0e-7 / 1.0e-7), for 10 to 20 % of the time of a launch.
+//
+// What bounds it: per code 5/8 (4/8 at 2 bits) of an operation of the half-rate pipe and half a packed multiply-add, 0.055 warp
 // instructions in all, against three dot products of four bytes (0.75 operations and 0.09 instructions) of the byte form in
 // gguf_dp.cu, which takes a pass over the weights per token (and is the faster one for one token: it has less to stage).  Structure, streams and clusters are those of qmv_mm.cu: a warp
 // takes tasks of sixteen rows and a run of steps (two Q4_K or four Q2_K blocks) through its own ring of asynchronous copies.
@@ -64,6 +69,11 @@ __device__ __forceinline__ uint32_t gm_mul(uint32_t a, uint32_t b) {
 __device__ __forceinline__ uint32_t gm_fma(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
     asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t gm_and_or(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
 __device__ __forceinline__ uint32_t gm_f16(float v) {
@@ -220,10 +230,10 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
             uint32_t amax = 0;
 #pragma unroll
             for (int j = 0; j < 8; ++j) amax = max(amax, __float_as_uint(f[j]) & 0x7fffffffu);
-            // E: biased exponent of the block's largest magnitude; below 2^-113 the block counts as zero, an infinity or NaN makes its
-            // factor NaN
-            const uint32_t e = __reduce_max_sync(0xffffffffu, amax) >> 23;
-            const bool live = e >= 14u && e < 255u;
+            // E: biased exponent of the block's largest magnitude, at least the one whose factor is a float (smaller blocks keep that
+            // scale); an infinity or NaN makes its factor NaN
+            const uint32_t e0 = __reduce_max_sync(0xffffffffu, amax) >> 23, e = max(e0, 14u);
+            const bool live = e0 < 255u;
             const float up = live ? __uint_as_float((267u - e) << 23) : 0.f;  // 2^(13 - (E - 127))
             uint32_t h[3][8];
 #pragma unroll
@@ -262,7 +272,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
                 for (int pl = 0; pl < 3; ++pl)
                     asm volatile("st.shared.u16 [%0], %1;" ::"r"(sums + b * sum_bytes + ((tok * 3 + pl) * 4 + tt) * 8 + at), "h"(static_cast<uint16_t>(hs[pl])) : "memory");
                 if (lane == 0) {
-                    const float factor = live ? __uint_as_float((e - 13u) << 23) : (e == 255u ? __uint_as_float(0x7fc00000u) : 0.f);
+                    const float factor = __uint_as_float(live ? (e - 13u) << 23 : 0x7fc00000u);
                     asm volatile("st.shared.f32 [%0], %1;" ::"r"(fac + (b * (cols / 3) + tok) * 4), "f"(factor) : "memory");
                 }
             }
@@ -275,7 +285,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
     uint32_t mk[4], magic;
 #pragma unroll
     for (int i = 0; i < 4; ++i) asm volatile("mov.u32 %0, %1;" : "=r"(mk[i]) : "r"(FMT == 4 ? (0x000f000fu << (4 * (i & 1))) : (0x00030003u << (2 * i))));
-    asm volatile("mov.u32 %0, 0x64646464;" : "=r"(magic));
+    asm volatile("mov.u32 %0, 0x64006400;" : "=r"(magic));  // (1024, 1024)
     // fragment column g of tile n is column min(8 n + g, cols - 1): the rest repeats the last one and is not stored
     uint32_t bcol[NT], scol[NT];
     uint32_t fcol[NT][2];
@@ -303,14 +313,14 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
         for (int step = prt * p.spt; step < end; ++step) {
             asm volatile("cp.async.wait_group %0;" ::"n"(kGmDepth - 1) : "memory");
             __syncwarp();
-            const uint32_t off = ((rg & odd) ^ (PIECE == 16 && FMT == 2 ? (s0 + step) & 1 : 0)) << 4;  // (rows 8 apart: the same offset)
-            const uint32_t r0 = at + rg * S::kPitch + off;
+            const uint32_t at_odd = ((rg & odd) ^ (PIECE == 16 && FMT == 2 ? (s0 + step) & 1 : 0)) << 4;  // (rows 8 apart: the same offset)
+            const uint32_t r0 = at + rg * S::kPitch + at_odd;
 #pragma unroll(FMT == 4 ? 1 : 4)
             for (int b = 0; b < S::kBlocks; ++b) {
                 const uint32_t bi = static_cast<uint32_t>(step * S::kBlocks + b);
                 constexpr int WORDS = FMT == 4 ? 8 : 4;
                 uint32_t cw[2][WORDS], mn[2][2], dm[2];
-                uint32_t sc[2][4];  // f16x2 scales of the lane's four sub-blocks, divided by their places
+                uint32_t sc[2][4], off[2][4];  // f16x2 scales of the lane's four sub-blocks, divided by their places; -1024 times that
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     const uint32_t blk = r0 + r * (8 * S::kPitch) + b * S::kBlock;
@@ -324,10 +334,10 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
                         // 6-bit scales and mins (quant.rs:88-96) of sub-blocks 2 (t / 2) + {0, 1} and 4 + 2 (t / 2) + {0, 1}
                         const int sh = 16 * (t >> 1);
                         const uint32_t a = hd[1] >> sh, m = hd[2] >> sh, hi = hd[3] >> sh;
-                        pair[0] = __byte_perm(a & 0x3f3fu, magic, 0x4140);
-                        pair[1] = __byte_perm((hi & 0x0f0fu) | ((a >> 2) & 0x3030u), magic, 0x4140);
-                        mn[r][0] = __byte_perm(m & 0x3f3fu, 0u, 0x4140);
-                        mn[r][1] = __byte_perm(((hi >> 4) & 0x0f0fu) | ((m >> 2) & 0x3030u), 0u, 0x4140);
+                        pair[0] = __byte_perm(a & 0x3f3fu, magic, 0x5150);
+                        pair[1] = __byte_perm((hi & 0x0f0fu) | ((a >> 2) & 0x3030u), magic, 0x5150);
+                        mn[r][0] = gm_fma(__byte_perm(m & 0x3f3fu, magic, 0x5150), 0x3c003c00u, 0xe400e400u);
+                        mn[r][1] = gm_fma(__byte_perm(((hi >> 4) & 0x0f0fu) | ((m >> 2) & 0x3030u), magic, 0x5150), 0x3c003c00u, 0xe400e400u);
                         // (1024 + s) - 1024, the second of a pair (high nibbles) divided by 16
 #pragma unroll
                         for (int i = 0; i < 2; ++i) pair[i] = gm_fma(pair[i], 0x2c003c00u, 0xd400e400u);
@@ -346,7 +356,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
                         for (int i = 0; i < 2; ++i) {
                             const uint32_t s = gm_lds32(blk + 8 * (t >> 1) + 4 * i) >> sh;  // scale bytes of fields 2 i, 2 i + 1
                             pair[i] = (s & 0x000f000fu) | 0x64006400u;
-                            mn[r][i] = (s >> 4) & 0x000f000fu;
+                            mn[r][i] = gm_fma(((s >> 4) & 0x000f000fu) | 0x64006400u, 0x3c003c00u, 0xe400e400u);
                         }
                         pair[0] = gm_fma(pair[0], 0x34003c00u, 0xdc00e400u);  // (s, s / 4)
                         pair[1] = gm_fma(pair[1], 0x24002c00u, 0xcc00d400u);  // (s / 16, s / 64)
@@ -355,13 +365,15 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
                     for (int i = 0; i < 2; ++i) {
                         sc[r][2 * i] = __byte_perm(pair[i], pair[i], 0x1010);
                         sc[r][2 * i + 1] = __byte_perm(pair[i], pair[i], 0x3232);
+                        off[r][2 * i] = gm_mul(sc[r][2 * i], 0xe400e400u);
+                        off[r][2 * i + 1] = gm_mul(sc[r][2 * i + 1], 0xe400e400u);
                     }
                 }
-                float c[NT][4], cm[NT][4];
+                float cm[NT][4], total[NT][4];
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) c[n][i] = cm[n][i] = 0.f;
+                    for (int i = 0; i < 4; ++i) cm[n][i] = total[n][i] = 0.f;
                     uint32_t bs[2];
                     asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(bs[0]), "=r"(bs[1]) : "r"(scol[n] + bi * sum_bytes));
                     gm_mma(cm[n], mn[0][0], mn[1][0], mn[0][1], mn[1][1], bs[0], bs[1]);
@@ -375,23 +387,25 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
                     for (int r = 0; r < 2; ++r)
 #pragma unroll
                         for (int f = 0; f < 2; ++f) {
-                            a[r][f][0] = gm_mul(cw[r][wi] & mk[f0 + f], sc[r][s_ + f]);
-                            a[r][f][1] = gm_mul((cw[r][wi] >> 8) & mk[f0 + f], sc[r][s_ + f]);
+                            a[r][f][0] = gm_fma(gm_and_or(cw[r][wi], mk[f0 + f], magic), sc[r][s_ + f], off[r][s_ + f]);
+                            a[r][f][1] = gm_fma(gm_and_or(cw[r][wi] >> 8, mk[f0 + f], magic), sc[r][s_ + f], off[r][s_ + f]);
                         }
 #pragma unroll
                     for (int n = 0; n < NT; ++n) {
+                        float c[4] = {0.f, 0.f, 0.f, 0.f};
                         uint32_t bf[4];
                         gm_lds128(bcol[n] + bi * blk_bytes + v * (cols * 64), bf);
-                        gm_mma(c[n], a[0][0][0], a[1][0][0], a[0][0][1], a[1][0][1], bf[0], bf[1]);
-                        gm_mma(c[n], a[0][1][0], a[1][1][0], a[0][1][1], a[1][1][1], bf[2], bf[3]);
+                        gm_mma(c, a[0][0][0], a[1][0][0], a[0][0][1], a[1][0][1], bf[0], bf[1]);
+                        gm_mma(c, a[0][1][0], a[1][1][0], a[0][1][1], a[1][1][1], bf[2], bf[3]);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) total[n][i] += c[i];
                     }
                 }
                 float d[2], dmin[2];
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     gm_half2(dm[r], d[r], dmin[r]);
-                    d[r] *= 16777216.f;        // the subnormals' 2^24
-                    dmin[r] *= -268435456.f;   // and the sums' 2^4
+                    dmin[r] *= -16.f;  // the sums' 2^4
                 }
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
@@ -400,7 +414,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
                         float f;
                         asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(fcol[n][j] + bi * (cols / 3 * 4)));
 #pragma unroll
-                        for (int r = 0; r < 2; ++r) acc[n][2 * r + j] = fmaf(fmaf(d[r], c[n][2 * r + j], dmin[r] * cm[n][2 * r + j]), f, acc[n][2 * r + j]);
+                        for (int r = 0; r < 2; ++r) acc[n][2 * r + j] = fmaf(fmaf(d[r], total[n][2 * r + j], dmin[r] * cm[n][2 * r + j]), f, acc[n][2 * r + j]);
                     }
                 }
             }

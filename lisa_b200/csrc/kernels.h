@@ -44,7 +44,7 @@ bool qmv_dp_supported(int64_t m, int64_t k, int count, const int64_t *n, int gro
 int qmv_dp(cudaStream_t stream, const void *x, int64_t m, int64_t k, int count, const uint32_t *const *w, const void *const *scales,
            const void *const *biases, const int64_t *n, int group_size, int bits, void *const *y, unsigned flags,
            const TcNormArgs *norm = nullptr);
-// qmv_mm.cu: the GEMV for up to eight rows in one pass on bf16 mma.sync; the same forms (group 64, 128)
+// qmv_mm.cu: the GEMV for up to eight rows in one pass on f16 mma.sync; the same forms (group 64, 128)
 bool qmv_mm_supported(int64_t m, int64_t k, int count, const int64_t *n, int group_size, int bits, bool fused);
 int qmv_mm(cudaStream_t stream, const void *x, int64_t m, int64_t k, int count, const uint32_t *const *w, const void *const *scales,
            const void *const *biases, const int64_t *n, int group_size, int bits, void *const *y, unsigned flags,
@@ -137,14 +137,15 @@ int gather_qmm_affine_multi(cudaStream_t stream, const void *x, int64_t rows, in
 int gguf_matvec(cudaStream_t stream, int format, const uint8_t *w, int64_t experts, int64_t rows, int64_t row_bytes,
                 const float *x, int64_t tokens, int64_t slots, const int32_t *ids, int64_t top_k, float *y);
 
-// gguf_mm.cu: the same, dense, for two tokens and more on mma.sync
+// gguf_mm.cu: the same, dense, on mma.sync; f32 sums of f32 activations
 bool gguf_mm_supported(int format, const void *w, int64_t tokens, int64_t rows, int64_t row_bytes);
 int gguf_mm(cudaStream_t stream, int format, const uint8_t *w, int64_t rows, int64_t row_bytes, const float *x, int64_t tokens, float *y);
 
-// gguf_dp.cu: the same for a few tokens or slots (zs = tokens, or tokens * top_k with ids) on byte dot products
-bool gguf_dp_supported(int format, const void *w, int64_t zs, int64_t rows, int64_t row_bytes, bool experts);
+// gguf_dp.cu: the same for one token, or a few slots (zs = tokens * top_k with ids), on byte dot products; exact: a grid of 2^-29 instead of
+// 2^-21 of a sub-block's largest activation
+bool gguf_dp_supported(int format, const void *w, int64_t zs, int64_t rows, int64_t row_bytes, bool experts, bool exact);
 int gguf_dp(cudaStream_t stream, int format, const uint8_t *w, int64_t experts, int64_t rows, int64_t row_bytes, const float *x, int64_t zs,
-            int64_t slots, const int32_t *ids, int64_t top_k, float *y);
+            int64_t slots, const int32_t *ids, int64_t top_k, float *y, bool exact);
 
 // moe.cu
 int moe_route(cudaStream_t stream, const float *logits, int64_t tokens, int64_t experts, int top_k, int32_t *idx,
