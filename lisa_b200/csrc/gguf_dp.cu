@@ -467,6 +467,7 @@ GdPlan gd_make_plan(int fmt, int64_t zs, int64_t rows, int64_t row_bytes, bool e
     for (int parts = 1; parts <= std::min(p.steps, 64); ++parts) {
         const int spt = (p.steps + parts - 1) / parts;
         if ((p.steps + spt - 1) / spt != parts) continue;
+        if (exact && spt != (p.steps + 15) / 16) continue;  // cut by the length of a row alone: a row has the same bits whatever the matrix and the slots
         const double cost = ((per * parts + kGdWarps - 1) / kGdWarps) * (spt + 0.1) + 0.01 * parts;
         if (cost < best) {
             best = cost;

@@ -30,6 +30,9 @@ namespace lisa {
 namespace {
 
 constexpr int kGmThreads = 512, kGmWarps = kGmThreads / 32, kGmDepth = 2;
+// The steps of a row are cut into up to eight leaves, by its length alone, and a row's sum is the balanced tree of theirs: clusters and tasks take
+// whole subtrees, so that a result has the same bits whatever the rows of the matrix, the tokens of the call and the launch.
+constexpr int gm_leaves(int steps) { return steps >= 8 ? 8 : steps >= 4 ? 4 : steps >= 2 ? 2 : 1; }
 
 struct GmParams {
     const uint8_t *w;
@@ -37,7 +40,7 @@ struct GmParams {
     float *y;
     long long row_bytes;
     int rows, k, blocks;     // rows of the matrix; k; 256-element blocks of a row
-    int steps, splits, max_steps, parts, spt, warps;
+    int steps, leaves, splits, parts, warps;
     int shares, base, extra;  // shares of the 16-row tiles per z; tiles of a share (the first `extra` one more)
     int tail_pieces;          // pieces of a row in its last step where that is ragged, else 0
     int tokens;               // tokens of the call (dense form)
@@ -130,13 +133,13 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
     const int job = static_cast<int>(blockIdx.x) / splits, z = job / p.shares, share = job - z * p.shares;
     const int qb = share * p.base + min(share, p.extra), tiles = p.base + (share < p.extra ? 1 : 0);
     const int s0 = CL ? rank * p.steps / splits : 0, steps = CL ? (rank + 1) * p.steps / splits - s0 : p.steps;
-    const int parts = CL ? (steps + p.spt - 1) / p.spt : p.parts;
+    const int parts = p.parts, pieces = splits * parts;  // of all CTAs of the row: 1, 2, 4 or 8
     const int cols = p.cols, set_tokens = cols / 3, ntok = min(set_tokens, p.tokens - z * set_tokens);
     const float *x = p.x + static_cast<size_t>(z) * set_tokens * p.k;
     float *y = p.y + static_cast<size_t>(z) * set_tokens * p.rows;
     if (CL) gm_cluster_arrive();
     const uint32_t frag = smem_u32(gm_smem), sums = frag + p.sums_at, fac = frag + p.fac_at;
-    float *part = reinterpret_cast<float *>(gm_smem + p.part_at);  // [rows of the share][splits][parts][tokens], in the first CTA
+    float *part = reinterpret_cast<float *>(gm_smem + p.part_at);  // [rows of the share][pieces][tokens], in the first CTA
     const uint32_t ring = frag + p.ring_at + warp * kGmDepth * S::kSlot;
 
     // ---- the stream (see qmv_mm.cu): copy h moves piece h * 32 + lane of the sixteen rows.  With 16-byte pieces a row keeps the offset
@@ -163,8 +166,8 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
             ahead.left = 0;
             return;
         }
-        const int step = s0 + ahead.part * p.spt, row0 = (qb + ahead.set) * 16;
-        ahead.left = min(p.spt, s0 + steps - step);
+        const int at = rank * parts + ahead.part, step = at * p.steps / pieces, row0 = (qb + ahead.set) * 16;
+        ahead.left = (at + 1) * p.steps / pieces - step;  // (at least one: pieces <= steps)
         ahead.ragged = p.tail_pieces && step + ahead.left == p.steps ? 1 : 0;
         ahead.shift = PIECE == 16 && FMT == 2 ? (step & 1) * 16 : 0;
         ahead.last = p.rows - 1 - row0;
@@ -306,142 +309,165 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
             ++prt;
         }
         if (prt >= parts) break;
-        float acc[NT][4];  // rows g, g + 8 x columns 2t, 2t + 1
+        // A lane's sums of the piece: rows g, g + 8 of tokens t, t + 4.  tree[l]: the subtree of 2^l leaves that waits for its right half, at the end the
+        // piece (in local memory, by runtime indices: registers are short in the loop over the steps).
+        constexpr int LT = (8 * NT / 3 + 3) / 4;
+        float tree[4][LT * 2];
+        const int leaves = p.leaves / pieces, leaf0 = (rank * parts + prt) * leaves;
+        int step = leaf0 * p.steps / p.leaves - s0;
+#pragma unroll 1
+        for (int leaf = 0; leaf < leaves; ++leaf) {
+            float acc[NT][4];  // rows g, g + 8 x columns 2t, 2t + 1
 #pragma unroll
-        for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-        const int end = min((prt + 1) * p.spt, steps);
-        for (int step = prt * p.spt; step < end; ++step) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(kGmDepth - 1) : "memory");
-            __syncwarp();
-            const uint32_t at_odd = ((rg & odd) ^ (PIECE == 16 && FMT == 2 ? (s0 + step) & 1 : 0)) << 4;  // (rows 8 apart: the same offset)
-            const uint32_t r0 = at + rg * S::kPitch + at_odd;
+            for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+            const int end = (leaf0 + leaf + 1) * p.steps / p.leaves - s0;
+#pragma unroll 1
+            for (; step < end; ++step) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kGmDepth - 1) : "memory");
+                __syncwarp();
+                const uint32_t at_odd = ((rg & odd) ^ (PIECE == 16 && FMT == 2 ? (s0 + step) & 1 : 0)) << 4;  // (rows 8 apart: the same offset)
+                const uint32_t r0 = at + rg * S::kPitch + at_odd;
 #pragma unroll(FMT == 4 ? 1 : 4)
-            for (int b = 0; b < S::kBlocks; ++b) {
-                const uint32_t bi = static_cast<uint32_t>(step * S::kBlocks + b);
-                constexpr int WORDS = FMT == 4 ? 8 : 4;
-                uint32_t cw[2][WORDS], mn[2][2], dm[2];
-                uint32_t sc[2][4], off[2][4];  // f16x2 scales of the lane's four sub-blocks, divided by their places; -1024 times that
+                for (int b = 0; b < S::kBlocks; ++b) {
+                    const uint32_t bi = static_cast<uint32_t>(step * S::kBlocks + b);
+                    constexpr int WORDS = FMT == 4 ? 8 : 4;
+                    uint32_t cw[2][WORDS], mn[2][2], dm[2];
+                    uint32_t sc[2][4], off[2][4];  // f16x2 scales of the lane's four sub-blocks, divided by their places; -1024 times that
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    const uint32_t blk = r0 + r * (8 * S::kPitch) + b * S::kBlock;
-                    uint32_t pair[2];
-                    if constexpr (FMT == 4) {
-                        uint32_t hd[4];
-                        gm_lds128(blk, hd);
-                        gm_lds128(blk + 16 + 16 * t, cw[r]);
-                        gm_lds128(blk + 80 + 16 * t, cw[r] + 4);
-                        dm[r] = hd[0];
-                        // 6-bit scales and mins (quant.rs:88-96) of sub-blocks 2 (t / 2) + {0, 1} and 4 + 2 (t / 2) + {0, 1}
-                        const int sh = 16 * (t >> 1);
-                        const uint32_t a = hd[1] >> sh, m = hd[2] >> sh, hi = hd[3] >> sh;
-                        pair[0] = __byte_perm(a & 0x3f3fu, magic, 0x5150);
-                        pair[1] = __byte_perm((hi & 0x0f0fu) | ((a >> 2) & 0x3030u), magic, 0x5150);
-                        mn[r][0] = gm_fma(__byte_perm(m & 0x3f3fu, magic, 0x5150), 0x3c003c00u, 0xe400e400u);
-                        mn[r][1] = gm_fma(__byte_perm(((hi >> 4) & 0x0f0fu) | ((m >> 2) & 0x3030u), magic, 0x5150), 0x3c003c00u, 0xe400e400u);
-                        // (1024 + s) - 1024, the second of a pair (high nibbles) divided by 16
+                    for (int r = 0; r < 2; ++r) {
+                        const uint32_t blk = r0 + r * (8 * S::kPitch) + b * S::kBlock;
+                        uint32_t pair[2];
+                        if constexpr (FMT == 4) {
+                            uint32_t hd[4];
+                            gm_lds128(blk, hd);
+                            gm_lds128(blk + 16 + 16 * t, cw[r]);
+                            gm_lds128(blk + 80 + 16 * t, cw[r] + 4);
+                            dm[r] = hd[0];
+                            // 6-bit scales and mins (quant.rs:88-96) of sub-blocks 2 (t / 2) + {0, 1} and 4 + 2 (t / 2) + {0, 1}
+                            const int sh = 16 * (t >> 1);
+                            const uint32_t a = hd[1] >> sh, m = hd[2] >> sh, hi = hd[3] >> sh;
+                            pair[0] = __byte_perm(a & 0x3f3fu, magic, 0x5150);
+                            pair[1] = __byte_perm((hi & 0x0f0fu) | ((a >> 2) & 0x3030u), magic, 0x5150);
+                            mn[r][0] = gm_fma(__byte_perm(m & 0x3f3fu, magic, 0x5150), 0x3c003c00u, 0xe400e400u);
+                            mn[r][1] = gm_fma(__byte_perm(((hi >> 4) & 0x0f0fu) | ((m >> 2) & 0x3030u), magic, 0x5150), 0x3c003c00u, 0xe400e400u);
+                            // (1024 + s) - 1024, the second of a pair (high nibbles) divided by 16
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) pair[i] = gm_fma(pair[i], 0x2c003c00u, 0xd400e400u);
-                    } else {
-                        // the block's codes start at word 4 + 21 b of the row: aligned vectors, the lane's four words in two of them
-                        constexpr int kAligned[4] = {16, 96, 176, 256}, kWord[4] = {0, 1, 2, 3};
-                        uint32_t v[8];
-                        const uint32_t vec = r0 + r * (8 * S::kPitch) + kAligned[b] + 16 * t;
-                        gm_lds128(vec, v);
-                        if (kWord[b]) gm_lds128(vec + 16, v + 4);
+                            for (int i = 0; i < 2; ++i) pair[i] = gm_fma(pair[i], 0x2c003c00u, 0xd400e400u);
+                        } else {
+                            // the block's codes start at word 4 + 21 b of the row: aligned vectors, the lane's four words in two of them
+                            constexpr int kAligned[4] = {16, 96, 176, 256}, kWord[4] = {0, 1, 2, 3};
+                            uint32_t v[8];
+                            const uint32_t vec = r0 + r * (8 * S::kPitch) + kAligned[b] + 16 * t;
+                            gm_lds128(vec, v);
+                            if (kWord[b]) gm_lds128(vec + 16, v + 4);
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) cw[r][i] = v[kWord[b] + i];
-                        dm[r] = gm_lds32(blk + 80);
-                        const int sh = 8 * (t & 1);
+                            for (int i = 0; i < 4; ++i) cw[r][i] = v[kWord[b] + i];
+                            dm[r] = gm_lds32(blk + 80);
+                            const int sh = 8 * (t & 1);
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const uint32_t s = gm_lds32(blk + 8 * (t >> 1) + 4 * i) >> sh;  // scale bytes of fields 2 i, 2 i + 1
+                                pair[i] = (s & 0x000f000fu) | 0x64006400u;
+                                mn[r][i] = gm_fma(((s >> 4) & 0x000f000fu) | 0x64006400u, 0x3c003c00u, 0xe400e400u);
+                            }
+                            pair[0] = gm_fma(pair[0], 0x34003c00u, 0xdc00e400u);  // (s, s / 4)
+                            pair[1] = gm_fma(pair[1], 0x24002c00u, 0xcc00d400u);  // (s / 16, s / 64)
+                        }
 #pragma unroll
                         for (int i = 0; i < 2; ++i) {
-                            const uint32_t s = gm_lds32(blk + 8 * (t >> 1) + 4 * i) >> sh;  // scale bytes of fields 2 i, 2 i + 1
-                            pair[i] = (s & 0x000f000fu) | 0x64006400u;
-                            mn[r][i] = gm_fma(((s >> 4) & 0x000f000fu) | 0x64006400u, 0x3c003c00u, 0xe400e400u);
+                            sc[r][2 * i] = __byte_perm(pair[i], pair[i], 0x1010);
+                            sc[r][2 * i + 1] = __byte_perm(pair[i], pair[i], 0x3232);
+                            off[r][2 * i] = gm_mul(sc[r][2 * i], 0xe400e400u);
+                            off[r][2 * i + 1] = gm_mul(sc[r][2 * i + 1], 0xe400e400u);
                         }
-                        pair[0] = gm_fma(pair[0], 0x34003c00u, 0xdc00e400u);  // (s, s / 4)
-                        pair[1] = gm_fma(pair[1], 0x24002c00u, 0xcc00d400u);  // (s / 16, s / 64)
                     }
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        sc[r][2 * i] = __byte_perm(pair[i], pair[i], 0x1010);
-                        sc[r][2 * i + 1] = __byte_perm(pair[i], pair[i], 0x3232);
-                        off[r][2 * i] = gm_mul(sc[r][2 * i], 0xe400e400u);
-                        off[r][2 * i + 1] = gm_mul(sc[r][2 * i + 1], 0xe400e400u);
-                    }
-                }
-                float cm[NT][4], total[NT][4];
-#pragma unroll
-                for (int n = 0; n < NT; ++n) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) cm[n][i] = total[n][i] = 0.f;
-                    uint32_t bs[2];
-                    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(bs[0]), "=r"(bs[1]) : "r"(scol[n] + bi * sum_bytes));
-                    gm_mma(cm[n], mn[0][0], mn[1][0], mn[0][1], mn[1][1], bs[0], bs[1]);
-                }
-#pragma unroll
-                for (int v = 0; v < 8; ++v) {
-                    // Q4_K: word v, low and high nibbles; Q2_K: word v / 2, fields 2 (v % 2) and + 1
-                    const int wi = FMT == 4 ? v : v >> 1, f0 = FMT == 4 ? 0 : 2 * (v & 1), s_ = FMT == 4 ? 2 * (v >> 2) : f0;
-                    uint32_t a[2][2][2];  // [row][field][bytes 0|2, 1|3]
-#pragma unroll
-                    for (int r = 0; r < 2; ++r)
-#pragma unroll
-                        for (int f = 0; f < 2; ++f) {
-                            a[r][f][0] = gm_fma(gm_and_or(cw[r][wi], mk[f0 + f], magic), sc[r][s_ + f], off[r][s_ + f]);
-                            a[r][f][1] = gm_fma(gm_and_or(cw[r][wi] >> 8, mk[f0 + f], magic), sc[r][s_ + f], off[r][s_ + f]);
-                        }
+                    float cm[NT][4], total[NT][4];
 #pragma unroll
                     for (int n = 0; n < NT; ++n) {
-                        float c[4] = {0.f, 0.f, 0.f, 0.f};
-                        uint32_t bf[4];
-                        gm_lds128(bcol[n] + bi * blk_bytes + v * (cols * 64), bf);
-                        gm_mma(c, a[0][0][0], a[1][0][0], a[0][0][1], a[1][0][1], bf[0], bf[1]);
-                        gm_mma(c, a[0][1][0], a[1][1][0], a[0][1][1], a[1][1][1], bf[2], bf[3]);
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) total[n][i] += c[i];
+                        for (int i = 0; i < 4; ++i) cm[n][i] = total[n][i] = 0.f;
+                        uint32_t bs[2];
+                        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(bs[0]), "=r"(bs[1]) : "r"(scol[n] + bi * sum_bytes));
+                        gm_mma(cm[n], mn[0][0], mn[1][0], mn[0][1], mn[1][1], bs[0], bs[1]);
+                    }
+#pragma unroll
+                    for (int v = 0; v < 8; ++v) {
+                        // Q4_K: word v, low and high nibbles; Q2_K: word v / 2, fields 2 (v % 2) and + 1
+                        const int wi = FMT == 4 ? v : v >> 1, f0 = FMT == 4 ? 0 : 2 * (v & 1), s_ = FMT == 4 ? 2 * (v >> 2) : f0;
+                        uint32_t a[2][2][2];  // [row][field][bytes 0|2, 1|3]
+#pragma unroll
+                        for (int r = 0; r < 2; ++r)
+#pragma unroll
+                            for (int f = 0; f < 2; ++f) {
+                                a[r][f][0] = gm_fma(gm_and_or(cw[r][wi], mk[f0 + f], magic), sc[r][s_ + f], off[r][s_ + f]);
+                                a[r][f][1] = gm_fma(gm_and_or(cw[r][wi] >> 8, mk[f0 + f], magic), sc[r][s_ + f], off[r][s_ + f]);
+                            }
+#pragma unroll
+                        for (int n = 0; n < NT; ++n) {
+                            float c[4] = {0.f, 0.f, 0.f, 0.f};
+                            uint32_t bf[4];
+                            gm_lds128(bcol[n] + bi * blk_bytes + v * (cols * 64), bf);
+                            gm_mma(c, a[0][0][0], a[1][0][0], a[0][0][1], a[1][0][1], bf[0], bf[1]);
+                            gm_mma(c, a[0][1][0], a[1][1][0], a[0][1][1], a[1][1][1], bf[2], bf[3]);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) total[n][i] += c[i];
+                        }
+                    }
+                    float d[2], dmin[2];
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        gm_half2(dm[r], d[r], dmin[r]);
+                        dmin[r] *= -16.f;  // the sums' 2^4
+                    }
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            float f;
+                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(fcol[n][j] + bi * (cols / 3 * 4)));
+#pragma unroll
+                            for (int r = 0; r < 2; ++r) acc[n][2 * r + j] = fmaf(fmaf(d[r], total[n][2 * r + j], dmin[r] * cm[n][2 * r + j]), f, acc[n][2 * r + j]);
+                        }
                     }
                 }
-                float d[2], dmin[2];
+                __syncwarp();
+                fetch();
+                at = at == ring ? ring + S::kSlot : ring;
+            }
+            // the three planes of a token lie in up to three lanes of the fragment row: their sum to lane (token % 4)
+            float sum[LT * 2];
+#pragma unroll
+            for (int k = 0; k < 8 * NT / 3; ++k) {
+                if (k >= ntok) break;
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                    gm_half2(dm[r], d[r], dmin[r]);
-                    dmin[r] *= -16.f;  // the sums' 2^4
-                }
+                    float v[3];
 #pragma unroll
-                for (int n = 0; n < NT; ++n) {
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        float f;
-                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(fcol[n][j] + bi * (cols / 3 * 4)));
-#pragma unroll
-                        for (int r = 0; r < 2; ++r) acc[n][2 * r + j] = fmaf(fmaf(d[r], total[n][2 * r + j], dmin[r] * cm[n][2 * r + j]), f, acc[n][2 * r + j]);
+                    for (int pl = 0; pl < 3; ++pl) {
+                        const int col = 3 * k + pl;  // tile col / 8, lane (col % 8) / 2, its value col % 2
+                        v[pl] = __shfl_sync(0xffffffffu, acc[col / 8][2 * r + (col & 1)], (lane & ~3) | ((col & 7) >> 1));
                     }
+                    if (t == (k & 3)) sum[k / 4 * 2 + r] = v[0] + (v[1] + v[2]);
                 }
             }
-            __syncwarp();
-            fetch();
-            at = at == ring ? ring + S::kSlot : ring;
+            int level = 0;
+#pragma unroll 1
+            for (; (leaf >> level) & 1; ++level)
+#pragma unroll
+                for (int i = 0; i < LT * 2; ++i) sum[i] = tree[level][i] + sum[i];
+#pragma unroll
+            for (int i = 0; i < LT * 2; ++i) tree[level][i] = sum[i];
         }
-        // the three planes of a token lie in up to three lanes of the fragment row: their sum to lane (token % 4)
+        const int top = 31 - __clz(leaves);
 #pragma unroll
-        for (int k = 0; k < 8 * NT / 3; ++k) {
-            if (k >= ntok) break;
+        for (int i = 0; i < LT; ++i)
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                float v[3];
-#pragma unroll
-                for (int pl = 0; pl < 3; ++pl) {
-                    const int col = 3 * k + pl;  // tile col / 8, lane (col % 8) / 2, its value col % 2
-                    v[pl] = __shfl_sync(0xffffffffu, acc[col / 8][2 * r + (col & 1)], (lane & ~3) | ((col & 7) >> 1));
+            for (int r = 0; r < 2; ++r)
+                if (4 * i + t < ntok) {
+                    float *to = part + ((set * 16 + r * 8 + rg) * pieces + rank * parts + prt) * set_tokens + 4 * i + t;
+                    if (CL) gm_st_cluster(to, 0, tree[top][i * 2 + r]);
+                    else *to = tree[top][i * 2 + r];
                 }
-                if (t == (k & 3)) {
-                    float *to = part + (((set * 16 + r * 8 + rg) * splits + rank) * p.parts + prt) * set_tokens + k;
-                    const float sum = v[0] + (v[1] + v[2]);
-                    if (CL) gm_st_cluster(to, 0, sum);
-                    else *to = sum;
-                }
-            }
-        }
         set += p.warps;
     }
     if (CL) {
@@ -452,16 +478,17 @@ __global__ void __launch_bounds__(kGmThreads, 1) gguf_mm_kernel(const GmParams p
         __syncthreads();
     }
 
-    // ---- sum of the parts in the order of k; store
+    // ---- the top of the tree; store
     for (int i = tid; i < tiles * 16 * ntok; i += kGmThreads) {
         const int tok = i / (tiles * 16), rr = i - tok * (tiles * 16), row = qb * 16 + rr;
         if (row >= p.rows) continue;
-        float tot = 0.f;
-        for (int r = 0; r < splits; ++r) {
-            const int cnt = CL ? ((r + 1) * p.steps / splits - r * p.steps / splits + p.spt - 1) / p.spt : p.parts;
-            for (int q = 0; q < cnt; ++q)
-                tot += part[((rr * splits + r) * p.parts + q) * set_tokens + tok];
-        }
+        const float *v = part + rr * pieces * set_tokens + tok;
+        auto two = [&](int i) { return v[i * set_tokens] + v[(i + 1) * set_tokens]; };
+        float tot;
+        if (pieces == 1) tot = v[0];
+        else if (pieces == 2) tot = two(0);
+        else if (pieces == 4) tot = two(0) + two(2);
+        else tot = (two(0) + two(2)) + (two(4) + two(6));
         y[static_cast<size_t>(tok) * p.rows + row] = tot;
     }
 }
@@ -512,60 +539,66 @@ GmPlan gm_make_plan(int fmt, int64_t tokens, int64_t rows, int64_t row_bytes) {
     p.blocks = static_cast<int>(nb);
     p.k = static_cast<int>(nb * 256);
     p.steps = static_cast<int>((nb + blocks - 1) / blocks);
+    p.leaves = gm_leaves(p.steps);
     pl.piece = row_bytes % 16 == 0 ? 16 : row_bytes % 8 == 0 ? 8 : 4;
     p.tail_pieces = nb % blocks ? static_cast<int>(nb % blocks) * block / pl.piece : 0;
     const int64_t tiles = (rows + 15) / 16;
     p.tokens = static_cast<int>(tokens);
     double best = 1e30;
     // Tokens of a column set: eight, five or two fill three, two or one column tiles; more tokens run as several sets of nearly the same
-    // size side by side (their weights meet in L2).
-    for (int most_tokens : {8, 5, 2}) {
-    const int64_t zs = (tokens + most_tokens - 1) / most_tokens, set = (tokens + zs - 1) / zs;
-    const int64_t cols = 3 * set;
-    const int nt = static_cast<int>((cols + 7) / 8);
-    for (int splits : {1, 2, 4, 8}) {
-        if (splits > p.steps) continue;
-        const int64_t at_once = splits == 1 ? sm_count() : gm_cluster_limit(splits);
-        const int64_t shares = std::min<int64_t>(tiles, std::max<int64_t>(1, at_once / zs));
-        const int per = static_cast<int>((tiles + shares - 1) / shares), most = (p.steps + splits - 1) / splits;
-        const int64_t rounds = (shares * zs + at_once - 1) / at_once;
-        const int64_t frag = static_cast<int64_t>(most) * blocks;
-        const int64_t sums_at = frag * 512 * cols, fac_at = sums_at + frag * 32 * cols, ring_at = (fac_at + frag * set * 4 + 127) & ~static_cast<int64_t>(127);
-        if (ring_at > max_smem_optin()) continue;
-        for (int warps : {16, 12, 8}) {
-            // time of a step: against sixteen warps; a column tile more costs a quarter
-            const double pace = (warps == 16 ? 1.0 : warps == 12 ? 0.85 : 0.7) * (0.75 + 0.25 * nt);
-            for (int parts = 1; parts <= std::min(most, 64); ++parts) {
-                const int spt = (most + parts - 1) / parts;
-                if ((most + spt - 1) / spt != parts) continue;
-                const int64_t part_at = ring_at + static_cast<int64_t>(warps) * kGmDepth * slot;
-                const int64_t bytes = part_at + static_cast<int64_t>(per) * 16 * splits * parts * set * 4;
-                if (bytes > max_smem_optin() - 2048) continue;
-                // ... and the staging of the activations (about a fifth of a step per block and token and warp)
-                const double cost = rounds * (((per * parts + warps - 1) / warps) * (spt + 0.1) * pace + 0.2 * frag * static_cast<double>(set) / kGmWarps) + 0.01 * parts +
-                                    (splits > 1 ? 0.5 * splits : 0);
-                if (cost < best) {
-                    best = cost;
-                    p.cols = static_cast<int>(cols);
-                    pl.nt = nt;
-                    p.splits = splits;
-                    p.warps = warps;
-                    p.parts = parts;
-                    p.spt = spt;
-                    p.max_steps = most;
-                    p.shares = static_cast<int>(shares);
-                    p.base = static_cast<int>(tiles / shares);
-                    p.extra = static_cast<int>(tiles % shares);
-                    p.sums_at = static_cast<int>(sums_at);
-                    p.fac_at = static_cast<int>(fac_at);
-                    p.ring_at = static_cast<int>(ring_at);
-                    p.part_at = static_cast<int>(part_at);
-                    pl.smem = static_cast<int>(bytes);
-                    pl.grid = static_cast<int>(zs * shares * splits);
+    // size side by side (their weights meet in L2).  Single tokens, and any number of CTAs, where nothing else fits: what fits depends on the
+    // length of a row alone.
+    for (int most_tokens : {8, 5, 2, 1}) {
+        const int64_t zs = (tokens + most_tokens - 1) / most_tokens, set = (tokens + zs - 1) / zs;
+        const int64_t cols = 3 * set;
+        const int nt = static_cast<int>((cols + 7) / 8);
+        const bool last = most_tokens == 1;
+        if (last && best < 1e30) break;
+        for (int splits : {1, 2, 4, 8}) {
+            if (splits > p.leaves) continue;
+            const int64_t at_once = splits == 1 ? sm_count() : gm_cluster_limit(splits);
+            const int most = (p.steps + splits - 1) / splits;
+            const int64_t frag = static_cast<int64_t>(most) * blocks;
+            const int64_t sums_at = frag * 512 * cols, fac_at = sums_at + frag * 32 * cols, ring_at = (fac_at + frag * set * 4 + 127) & ~static_cast<int64_t>(127);
+            if (ring_at > max_smem_optin()) continue;
+            // CTAs that run at a time, and two or four times as many, whose partial sums take less room
+            int64_t shares = std::min<int64_t>(tiles, std::max<int64_t>(1, at_once / zs));
+            for (int turn = 0;; ++turn, shares = std::min(tiles, 2 * shares)) {
+                const int64_t per = (tiles + shares - 1) / shares, rounds = (shares * zs + at_once - 1) / at_once;
+                bool fits = false;
+                for (int warps : {16, 12, 8}) {
+                    // time of a step: against sixteen warps and one column tile (three of them spill)
+                    const double pace = (warps == 16 ? 1.0 : warps == 12 ? 0.85 : 0.7) * (nt == 1 ? 1.0 : nt == 2 ? 1.25 : 2.2);
+                    for (int parts = 1; parts * splits <= p.leaves; parts *= 2) {
+                        const int64_t part_at = ring_at + static_cast<int64_t>(warps) * kGmDepth * slot;
+                        const int64_t bytes = part_at + per * 16 * splits * parts * set * 4;
+                        if (bytes > max_smem_optin() - 2048) continue;
+                        fits = true;
+                        // ... the staging of the activations (about a fifth of a step per block and token and warp), and five steps for a CTA's start
+                        const double cost = rounds * (((per * parts + warps - 1) / warps) * (static_cast<double>(most) / parts + 0.1) * pace + 0.2 * frag * static_cast<double>(set) / kGmWarps + 5.0) +
+                                            0.01 * parts + (splits > 1 ? 0.5 * splits : 0);
+                        if (cost < best) {
+                            best = cost;
+                            p.cols = static_cast<int>(cols);
+                            pl.nt = nt;
+                            p.splits = splits;
+                            p.warps = warps;
+                            p.parts = parts;
+                            p.shares = static_cast<int>(shares);
+                            p.base = static_cast<int>(tiles / shares);
+                            p.extra = static_cast<int>(tiles % shares);
+                            p.sums_at = static_cast<int>(sums_at);
+                            p.fac_at = static_cast<int>(fac_at);
+                            p.ring_at = static_cast<int>(ring_at);
+                            p.part_at = static_cast<int>(part_at);
+                            pl.smem = static_cast<int>(bytes);
+                            pl.grid = static_cast<int>(zs * shares * splits);
+                        }
+                    }
                 }
+                if (shares == tiles || (turn >= 2 && (fits || !last))) break;
             }
         }
-    }
     }
     pl.ok = best < 1e30;
     return pl;
@@ -610,9 +643,9 @@ int gm_launch(cudaStream_t stream, const GmPlan &pl) {
 
 }  // namespace
 
-// Q4_K and Q2_K; up to 4096 tokens (matrices that the tensor-core product does not take come here with any number).
+// Q4_K and Q2_K, any number of tokens (matrices that the tensor-core product does not take come here with all of theirs).
 bool gguf_mm_supported(int format, const void *w, int64_t tokens, int64_t rows, int64_t row_bytes) {
-    if ((format != LISA_GGUF_Q4_K && format != LISA_GGUF_Q2_K) || tokens < 1 || tokens > 4096) return false;
+    if ((format != LISA_GGUF_Q4_K && format != LISA_GGUF_Q2_K) || tokens < 1 || tokens > 65535) return false;
     GmPlan pl;
     if (!gm_plan(format == LISA_GGUF_Q4_K ? 4 : 2, tokens, rows, row_bytes, pl)) return false;
     return (reinterpret_cast<uintptr_t>(w) & static_cast<uintptr_t>(pl.piece - 1)) == 0;

@@ -137,12 +137,12 @@ int gather_qmm_affine_multi(cudaStream_t stream, const void *x, int64_t rows, in
 int gguf_matvec(cudaStream_t stream, int format, const uint8_t *w, int64_t experts, int64_t rows, int64_t row_bytes,
                 const float *x, int64_t tokens, int64_t slots, const int32_t *ids, int64_t top_k, float *y);
 
-// gguf_mm.cu: the same, dense, on mma.sync; f32 sums of f32 activations
+// gguf_mm.cu: the same, dense, on mma.sync; f32 sums of f32 activations, bits by the length of a row alone
 bool gguf_mm_supported(int format, const void *w, int64_t tokens, int64_t rows, int64_t row_bytes);
 int gguf_mm(cudaStream_t stream, int format, const uint8_t *w, int64_t rows, int64_t row_bytes, const float *x, int64_t tokens, float *y);
 
 // gguf_dp.cu: the same for one token, or a few slots (zs = tokens * top_k with ids), on byte dot products; exact: a grid of 2^-29 instead of
-// 2^-21 of a sub-block's largest activation
+// 2^-21 of a sub-block's largest activation, and bits by the length of a row alone
 bool gguf_dp_supported(int format, const void *w, int64_t zs, int64_t rows, int64_t row_bytes, bool experts, bool exact);
 int gguf_dp(cudaStream_t stream, int format, const uint8_t *w, int64_t experts, int64_t rows, int64_t row_bytes, const float *x, int64_t zs,
             int64_t slots, const int32_t *ids, int64_t top_k, float *y, bool exact);

@@ -1,4 +1,4 @@
-"""GGUF matvecs of f32 activations: sums as good as f32 ones."""
+"""GGUF matvecs of f32 activations: sums as good as f32 ones, and a row's bits by its length alone."""
 import numpy as np
 import pytest
 import torch
@@ -46,6 +46,34 @@ def test_expert_error_against_f64_is_that_of_f32_sums(cuda, name, fmt, experts, 
     truth = np.einsum("tk,tjrk->tjr", x[:, 0].astype(np.float64), O.gguf_decode(fmt, w).reshape(experts, rows, k).astype(np.float64)[ids])
     _, l2 = util.parity(ops.expert_matvec(name, dev_u8(w, cuda), dev_f32(x, cuda), torch.from_numpy(ids).to(cuda)).cpu().numpy(), truth)
     assert l2 <= 1.6e-7, l2
+
+
+@pytest.mark.parametrize("name,fmt,k", [("Q2K", O.Q2_K, 256), ("Q2K", O.Q2_K, 2048), ("Q2K", O.Q2_K, 2816), ("Q2K", O.Q2_K, 18432), ("Q4K", O.Q4_K, 768), ("Q4K", O.Q4_K, 2048),
+                                        ("Q4K", O.Q4_K, 7168), ("Q4K", O.Q4_K, 18432)])
+def test_bits_of_a_row_do_not_depend_on_the_matrix_or_the_batch(cuda, name, fmt, k):
+    """A shard of the rows, or some of the tokens, gives what the whole gives, bit for bit: plans differ in clusters, tasks, token sets and rounds."""
+    rng = np.random.default_rng(k)
+    rows, tokens = 9216, 24
+    w = dev_u8(util.gguf_weights(rng, fmt, rows, k), cuda)
+    x = dev_f32(rng.normal(0, 1, size=(tokens, k)).astype(np.float32), cuda)
+    full = ops.packed_matvec(name, w, x)
+    for r0, r1 in ((0, 8), (4608, 9216), (1024, 3496)):
+        part = w[r0:r1].contiguous()
+        for t0, t1 in ((0, 24), (3, 5), (7, 10), (11, 16), (16, 24)):
+            assert torch.equal(ops.packed_matvec(name, part, x[t0:t1].contiguous()), full[t0:t1, r0:r1]), (r0, r1, t0, t1)
+    if k % 1024 and name == "Q2K":  # (a single token of whole stages is on the grid of the header)
+        assert torch.equal(ops.packed_matvec(name, w[:2304].contiguous(), x[9:10].contiguous()), full[9:10, :2304])
+
+
+def test_bits_of_an_expert_row_do_not_depend_on_the_slots(cuda):
+    rng = np.random.default_rng(5)
+    experts, rows, k, tokens, top_k = 6, 512, 2304, 20, 3
+    w = dev_u8(util.gguf_weights(rng, O.Q2_K, rows, k, experts=experts), cuda)
+    x = dev_f32(rng.normal(0, 1, size=(tokens, 1, k)).astype(np.float32), cuda)
+    ids = torch.from_numpy(rng.integers(0, experts, size=(tokens, top_k)).astype(np.int32)).to(cuda)
+    full = ops.expert_matvec("Q2K", w, x, ids)
+    assert torch.equal(ops.expert_matvec("Q2K", w, x[4:5].contiguous(), ids[4:5].contiguous()), full[4:5])
+    assert torch.equal(ops.expert_matvec("Q2K", w[:, 64:128].contiguous(), x, ids), full[..., 64:128])
 
 
 def test_small_activations_are_not_zeros(cuda):
