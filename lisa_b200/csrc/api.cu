@@ -791,6 +791,7 @@ int lisa_cuda_moe_block(lisa_stream_t stream, const void *x, const float *logits
     if (tokens > (1 << 24)) return fail(LISA_ERR_BAD_ARG, "moe_block: bad token count");
     const int64_t slots = tokens * top_k;
     const bool per_slot = slots < decode_slots;
+    if (per_slot && slots > (1 << 24)) return fail(LISA_ERR_BAD_ARG, "moe_block: bad slot count");
     const uint32_t *w3[3] = {wg, wu, wd};
     const void *s3[3] = {sg, su, sd}, *b3[3] = {bg, bu, bd};
     bool aligned = aligned16(x);

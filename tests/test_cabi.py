@@ -137,6 +137,7 @@ def test_moe_block_rejections(lib):
         assert call(limit, e=2048) == _cabi.ERR_LIMIT
         assert call(limit, e=1024, hidden=1 << 18, inter=1 << 17) == _cabi.ERR_OVERFLOW  # experts * n * k
         assert call(limit, ws=None) == _cabi.ERR_WORKSPACE and call(limit, wsb=64) == _cabi.ERR_WORKSPACE
+    assert call(1 << 40, tokens=1 << 23) == _cabi.ERR_BAD_ARG       # moe_gate_up_act's limit on slots
     assert lib.lisa_cuda_launch_count() == before
 
 
