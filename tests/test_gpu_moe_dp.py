@@ -1,11 +1,12 @@
-"""The routed block of a few tokens (moe_dp.cu) against the sorted chain, at the edges of its tiling."""
+"""The routed block of a few tokens (moe_dp.cu) against the oracle's block, at the edges of its tiling."""
 import numpy as np
 import pytest
 
 from lisa_b200 import ops
 from lisa_b200.quant import QuantizedLinear, SwitchGlu
+from oracle import oracle as O
 from tests import util
-from tests.gpu_util import dev_bf16, dev_f32, dev_u32
+from tests.gpu_util import dev_bf16, dev_f32, dev_u32, host_bf16_bits
 
 pytestmark = pytest.mark.gpu
 
@@ -17,20 +18,15 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("tokens", [1, 2])
 def test_edges(cuda, experts, top_k, hidden, inter, bits, gs, tokens):
     rng = np.random.default_rng(experts + top_k + hidden + inter + bits + gs + tokens)
-    shapes = [(inter, hidden), (inter, hidden), (hidden, inter)]
-    lins = [QuantizedLinear(*(f(a, cuda) for f, a in zip((dev_u32, dev_bf16, dev_bf16), util.affine_weights(rng, n, k, bits, gs, experts=experts))), gs, bits)
-            for n, k in shapes]
-    block = SwitchGlu(*lins, top_k)
-    x = dev_bf16(util.activations(rng, tokens, hidden), cuda)
+    host = [util.affine_weights(rng, n, k, bits, gs, experts=experts) for n, k in ((inter, hidden), (inter, hidden), (hidden, inter))]
+    block = SwitchGlu(*[QuantizedLinear(dev_u32(w, cuda), dev_bf16(s, cuda), dev_bf16(b, cuda), gs, bits) for w, s, b in host], top_k)
+    x = util.activations(rng, tokens, hidden)
     logits = rng.normal(size=(tokens, experts)).astype(np.float32)
     logits[0, 1] = logits[0, 0]  # a tie: the lower index first
-    tl = dev_f32(logits, cuda)
-    fast = block.forward(x, tl).float()
-    old = SwitchGlu.DECODE_SLOTS
-    try:
-        SwitchGlu.DECODE_SLOTS = 0
-        chain = block.forward(x, tl).float()
-    finally:
-        SwitchGlu.DECODE_SLOTS = old
-    assert float((fast - chain).abs().max()) <= 2.0 ** -6 * float(chain.abs().max())
+    got = O.bf16_to_f32(host_bf16_bits(block.forward(dev_bf16(x, cuda), dev_f32(logits, cuda))))
+    want, _ = O.moe_forward(x, logits, *host, top_k, gs, bits, round_weight_bf16=False)
+    err, l2 = util.parity(got, O.bf16_to_f32(want))
+    # gate, up, their product, down and the fold are rounded to bf16 on both sides: where a sum in another order falls to the other side, down's row and the
+    # fold move by an ulp, 2^-7 each at most; few do, so that the norm of the differences is below that of one rounding (2^-9 to each side)
+    assert err <= 2.0 ** -6 and l2 <= 2.0 ** -8, (err, l2)
     assert ops.device_status() == 0
