@@ -50,12 +50,13 @@ typedef enum lisa_gguf_format { LISA_GGUF_Q2_K = 10, LISA_GGUF_Q4_K = 12, LISA_G
 /* Dispatch overrides for lisa_cuda_quantized_matmul_ex. */
 enum {
     LISA_FLAG_NONE = 0,
-    LISA_FLAG_FORCE_QMV = 1 << 0,     /* mma.sync streaming kernel (staged ring) */
+    LISA_FLAG_FORCE_QMV = 1 << 0,     /* bf16 mma.sync streaming kernel (staged ring) */
     LISA_FLAG_FORCE_QMV_SIMPLE = 1 << 1, /* CUDA-core generic kernel (direct loads) */
     LISA_FLAG_FORCE_QMM = 1 << 2,     /* tcgen05 tensor-core kernel */
     LISA_FLAG_PDL = 1 << 3,           /* launch with programmatic stream serialization: the
-                                         kernel prefetches weights before waiting on the
-                                         previous kernel in the stream */
+                                         kernel prefetches weights (packed words, scales, biases,
+                                         a norm's weight) before waiting on the previous kernel in
+                                         the stream, which must not be what writes them */
     LISA_FLAG_FORCE_QMV_TC = 1 << 4,  /* streaming kernel with the unpacked weights in tensor memory
                                          (tcgen05): fail instead of falling back when the shape is
                                          not supported */
@@ -83,18 +84,26 @@ int lisa_cuda_clear_device_status(void);
  *   y [m,n] dtype.  m >= 1.  Like the reference: transpose must be non-zero and
  *   biases non-null (array_ops.rs:387-392).  bits in {2,4,8}, group_size in
  *   {32,64,128}, dtype LISA_BF16, or LISA_F16 / LISA_F32 (x, scales, biases and y all in it, as the
- *   reference casts them to the promoted dtype, array_ops.rs:398-404; these two, and 8-bit weights -- the
- *   lm-head case -- run on generic weight-streaming kernels at every row count; the other entry points of
+ *   reference casts them to the promoted dtype, array_ops.rs:398-404; these two run on a generic
+ *   weight-streaming kernel at every row count; the other entry points of
  *   this header are bf16 only).  Dispatch by m mirrors array_ops.rs:405-488:
- *   up to 8 rows stream the weights once (group size 64: the tensor-memory GEMV; other group sizes: the
- *   bf16 mma.sync or the generic kernel), more rows run the tcgen05 GEMM.
- *   Numerics of the group-64 GEMV: products and sums are exact integers, but the activations of a (row of
+ *   up to 8 rows stream the weights (one and two rows: byte dot products; three to eight, except group size
+ *   32 and 8-bit codes of other group sizes than 64: f16 mma.sync; shapes that these do not take: the
+ *   tensor-memory, bf16 mma.sync and generic kernels), more rows run the tcgen05 GEMM (8-bit weights: the
+ *   generic kernel).
+ *   Numerics of one and two rows of 2- and 4-bit codes with group size 64 (and of LISA_FLAG_FORCE_QMV_TC at
+ *   up to eight): products and sums are exact integers, but the activations of a (row of
  *   x, 64-k group) are first put on an integer grid of 2^-13 of the group's largest power of two (two
  *   signed bytes), so an element is off by at most 2^-14 of the group's largest magnitude; bf16
  *   activations within 2^-6 of that maximum are exact.  For Gaussian-like activations this is below the
  *   bf16 rounding of the output; a group with one element 2^10 times the rest loses the rest to about
  *   10 %.  LISA_FLAG_FORCE_QMV_I8 selects a kernel that adds a third byte (2^-22) for such groups,
- *   LISA_FLAG_FORCE_QMV one that keeps the bf16 activations exactly. */
+ *   LISA_FLAG_FORCE_QMV one that keeps the bf16 activations exactly.  8-bit codes, the other group sizes
+ *   and three to eight rows see the activations as they are (within 2^-30 of the group's largest).  A
+ *   non-finite activation makes its row of y NaN there, where the generic kernel's sums can end as an
+ *   infinity.
+ *   A row of a call of three to eight rows is not bit for bit what a one-row call gives (another kernel,
+ *   another order of the sums): lisa_cuda_quantized_matmul_serial_rows is the call for that. */
 int lisa_cuda_quantized_matmul(lisa_stream_t stream, const void *x, int64_t m, int64_t k,
                                const uint32_t *w, const void *scales, const void *biases,
                                int64_t n, int transpose, int group_size, int bits, int dtype,
@@ -116,8 +125,8 @@ int lisa_cuda_quantized_matmul_serial_rows(lisa_stream_t stream, const void *x, 
  * (crates/lisa-engine/src/models/qwen4/attention.rs:111-128 calls the three `forward(x)` one after
  * another) or gate_proj | up_proj of an MLP.  Linear i is (w[i], scales[i], biases[i]) with n[i]
  * output rows and writes its own [m, n[i]] output y[i]; results are those of `count` calls of
- * lisa_cuda_quantized_matmul within the f32 summation order.  For m <= 8 and shapes the
- * tensor-memory GEMV takes this is ONE launch (a decode launch costs microseconds whatever its size);
+ * lisa_cuda_quantized_matmul within the f32 summation order.  For m <= 8 and shapes a
+ * streaming kernel takes this is ONE launch (a decode launch costs microseconds whatever its size);
  * for more than 8 rows it is one tensor-core GEMM launch whose row tiles cover all the linears (small
  * ones no longer leave most SMs idle); otherwise the linears run one after another through the
  * dispatch of lisa_cuda_quantized_matmul. */
@@ -159,7 +168,7 @@ int lisa_cuda_quantized_matmul_allgather(lisa_stream_t stream, const void *x, in
  *   normed = dtype(norm_weight * dtype(f32(sum) * inv)),  inv = 1 / sqrt(mean(sum^2) + eps) in f32, per row
  *   y[i]   = normed . dequant(w[i])^T
  * The three roundings (sum, the product with inv, the product with the weight) are the reference's.  With up to 8
- * rows and shapes the tensor-memory kernel takes, add and norm run inside its activation staging: one launch, and
+ * rows of group size 64, 2- or 4-bit, add and norm run inside the linears' activation staging: one launch, and
  * `normed` may be null.  Every other shape runs lisa_cuda_add_rmsnorm and then the linears, and needs `normed`
  * (LISA_ERR_WORKSPACE without it).  norm_weight: dtype [k].  k a multiple of 8. */
 int lisa_cuda_quantized_matmul_addnorm(lisa_stream_t stream, const void *x, const void *residual, const void *norm_weight, float eps,
@@ -169,8 +178,9 @@ int lisa_cuda_quantized_matmul_addnorm(lisa_stream_t stream, const void *x, cons
 /* SwiGLU in front of a linear (the down projection of an MLP reading its gate and up outputs):
  *   act = dtype(dtype(gate * dtype(sigmoid(gate))) * up)  (crates/lisa-mlx/src/shaders/common/exact_header.metal:2-11)
  *   y   = act . dequant(w)^T
- * With up to 8 rows and shapes the tensor-memory kernel takes, the activation is formed in its staging: one
- * launch, `act` may be null (if given, it receives the activation rows).  Other shapes run lisa_cuda_swiglu and the
+ * With up to 8 rows of group size 64, 2- or 4-bit, the activation is formed in the linear's staging: one
+ * launch, `act` may be null (if given, it receives the activation rows, which three to eight rows then form by a launch of their
+ * own: faster than in every CTA's staging).  Other shapes run lisa_cuda_swiglu and the
  * ordinary dispatch and need `act` (LISA_ERR_WORKSPACE without it).  gate, up: dtype [m, k]. */
 int lisa_cuda_quantized_matmul_swiglu(lisa_stream_t stream, const void *gate, const void *up, int64_t m, int64_t k, const uint32_t *w,
                                       const void *scales, const void *biases, int64_t n, int transpose, int group_size, int bits,
@@ -244,9 +254,12 @@ int lisa_cuda_gather_qmm_siblings(lisa_stream_t stream, const void *x, int64_t r
 /* deepseek41::packed_matvec(format, weights, input), crates/lisa-mlx/src/models/deepseek41.rs:93-110.
  * w uint8 [rows, row_bytes] of GGUF blocks; x f32 [tokens, K], K = row_bytes/block*256;
  * y f32 [tokens, rows].  Same limits: rows % 8 == 0, row_bytes % block == 0,
- * 1 <= tokens <= 65535 (deepseek41.rs:50-65,100-101).  Formats: Q2_K (84-byte blocks), Q4_K (144), Q5_K (176);
- * one or two tokens of Q4_K and one token of Q2_K (rows of whole 336-byte groups) run through the tensor-memory
- * kernel, everything else one warp per row; both are exact on inputs whose products and sums are exact. */
+ * 1 <= tokens <= 65535 (deepseek41.rs:50-65,100-101).  Formats: Q2_K (84-byte blocks), Q4_K (144), Q5_K (176).
+ * One token of Q4_K, or of Q2_K with rows of whole 336-byte groups, runs on byte dot products: activations on a grid of
+ * 2^-21 of the largest power of two of their sub-block (16 or 32 elements).  Everything else sees f32 activations (Q4_K and
+ * Q2_K on mma.sync, each as the sum of three f16, with sums as good as f32 ones; Q5_K and odd addresses one warp per row), and
+ * a row's result there does not depend on the other rows or tokens: a shard of the matrix gives the same bits.  All are
+ * exact on inputs whose products and sums are exact.  A non-finite activation makes the row's results NaN. */
 int lisa_cuda_gguf_packed_matvec(lisa_stream_t stream, int format, const uint8_t *w, int64_t rows,
                                  int64_t row_bytes, const float *x, int64_t tokens, float *y);
 
@@ -277,7 +290,8 @@ int lisa_cuda_gguf_packed_matmul(lisa_stream_t stream, int format, const uint8_t
 /* deepseek41::expert_matvec(format, weights, input, ids), deepseek41.rs:204-283.
  * w uint8 [experts, rows, row_bytes]; x f32 [tokens, slots, K], slots in {1, top_k};
  * ids int32 [tokens, top_k], top_k <= 32; y f32 [tokens, top_k, rows].
- * An id < 0 or >= experts writes zeros without touching weight memory. */
+ * An id < 0 or >= experts writes zeros without touching weight memory.  Up to 256 slots (tokens * top_k) of Q4_K, or of Q2_K
+ * with rows of whole 336-byte groups, are on the grid of lisa_cuda_gguf_packed_matvec; other calls see f32 activations. */
 int lisa_cuda_gguf_expert_matvec(lisa_stream_t stream, int format, const uint8_t *w,
                                  int64_t experts, int64_t rows, int64_t row_bytes, const float *x,
                                  int64_t tokens, int64_t slots, const int32_t *ids, int64_t top_k,
@@ -352,8 +366,10 @@ int lisa_cuda_moe_down_combine(lisa_stream_t stream, const void *act, const int3
 
 /* The whole routed block (SparseMoeBlock::forward without its shared expert, crates/lisa-engine/src/models/qwen4/
  * moe.rs:116-350,352-481) as one call: route, then below `decode_slots` (token, expert) slots gate_up_act and
- * down_combine, from it on sort, gate | up, SwiGLU, down and combine: what the calls above give one after another, bit for
- * bit.  logits f32 [tokens, experts]; Wg, Wu [experts, inter, hidden * bits / 32], Wd [experts, hidden, inter * bits / 32];
+ * down_combine, from it on sort, gate | up, SwiGLU, down and combine: what the calls above give one after another, with
+ * their rounding points (every matmul result, SwiGLU step and the fold to bf16) and the activations as they are.  From
+ * `decode_slots` on it has their bits; below it the sums of the two products may run in another order than theirs, so that a
+ * rounding can fall the other way.  logits f32 [tokens, experts]; Wg, Wu [experts, inter, hidden * bits / 32], Wd [experts, hidden, inter * bits / 32];
  * out bf16 [tokens, hidden].  The workspace (16-byte aligned) holds everything between the steps. */
 size_t lisa_cuda_moe_block_workspace_bytes(int64_t tokens, int64_t experts, int top_k, int64_t hidden, int64_t inter);
 int lisa_cuda_moe_block(lisa_stream_t stream, const void *x, const float *logits, int64_t tokens, int64_t experts, int top_k,

@@ -103,11 +103,11 @@ static int check_affine(const char *op, const void *x, int64_t m, int64_t k, con
     return LISA_OK;
 }
 
-// Row count from which the tensor-core GEMM takes over from the weight-streaming kernel.
-// The reference switches at qmv_batch_limit (crates/lisa-mlx/src/jit/matmul.rs:1873-1881).  Here the
-// streaming kernel takes up to 8 rows in one pass over the weights while their activations fit its
+// Row count from which the tensor-core GEMM takes over from the older weight-streaming kernels, where qmv_dp and qmv_mm do not apply.
+// The reference switches at qmv_batch_limit (crates/lisa-mlx/src/jit/matmul.rs:1873-1881).  These
+// kernels take up to 8 rows in one pass over the weights while their activations fit the
 // shared-memory staging (m * k <= 8 * 9728, measured crossover); a GEMM CTA costs the same for any
-// tile of up to 256 rows, so it wins as soon as the streaming kernel would need a second pass.
+// tile of up to 256 rows, so it wins as soon as they would need a second pass.
 static const int64_t kQmvMaxRows = 8;
 static const int64_t kQmvMaxStaged = 8 * 9728;
 static bool prefer_qmv(int64_t m, int64_t k, bool tc_ok) {
@@ -116,9 +116,9 @@ static bool prefer_qmv(int64_t m, int64_t k, bool tc_ok) {
     return m <= kQmvMaxRows && (m <= 4 || m * k <= kQmvMaxStaged);
 }
 
-// Which weight-streaming kernel takes a call that both support: the tensor-memory kernel (measured faster on
-// every decode shape of the 4-bit stack), the integer mma.sync kernel when the environment says
-// LISA_QMV_KERNEL=i8 (read once; for side-by-side measurements) or LISA_FLAG_FORCE_QMV_I8 is given.
+// The integer mma.sync kernel takes the calls that it supports when the environment says LISA_QMV_KERNEL=i8 (read once; for
+// side-by-side measurements) or LISA_FLAG_FORCE_QMV_I8 is given.  Otherwise: qmv_dp for one and two rows, qmv_mm for three to
+// eight, and for the shapes which those leave (an odd number of groups, rows too long for shared memory) the tensor-memory kernel.
 static bool prefer_i8() {
     static const bool v = []() {
         const char *e = getenv("LISA_QMV_KERNEL");

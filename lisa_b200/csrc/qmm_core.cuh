@@ -11,13 +11,13 @@ namespace lisa {
 constexpr int kBN = 128;        // weight rows per CTA (MMA M)
 constexpr int kWideBt = 384;    // the tall token tile (template WIDE)
 constexpr int kBK = 64;         // k per MMA stage: 64 bf16 = one 128-byte swizzle row
-constexpr int kStages = 5;      // operand ring: stage s = activation tile in shared memory + A tile in tensor memory
+constexpr int kStages = 5;      // operand ring of the one-CTA form: stage s = activation tile in shared memory + A tile in tensor memory
 constexpr int kWpStages = 4;    // packed-weight ring: loads run a whole ring (12+ k-blocks) ahead of their use
 constexpr int kQ4kBlock = 144;  // GGUF Q4_K: bytes of a 256-element block = one packed stage row (4 k-blocks)
 constexpr int kQ2kBlock = 84;   // GGUF Q2_K: bytes of a block; a packed stage row is four of them (16 k-blocks)
 constexpr int kACols = kBK / 2; // one k-block of A: 64 bf16 per lane = 32 columns
-constexpr int kDequantWarps = 16;  // two sets of 8 warps (even / odd k-blocks); 2 threads per weight row, 32 codes each
-constexpr int kWarpsPerKb = kDequantWarps / 2;
+constexpr int kDequantWarps = 16;  // pairs: four sets of 4 warps, a thread per weight row; one CTA: two sets of 8 (even / odd k-blocks), two threads per row
+constexpr int kWarpsPerKb = kDequantWarps / 2;  // (the one-CTA form)
 constexpr int kThreads = (2 + kDequantWarps) * 32;
 constexpr int kWpBytes = kBN * 128;       // 16 KiB
 
@@ -274,10 +274,10 @@ struct QmmDecode {
             }
         } else {
             // bf16(q * s + b) for two codes at a time: a code goes to the low mantissa bits of 128.0 (one LOP3 for the codes 16 bits apart),
-            // minus 128 (exact), times s plus b with one rounding; bytes are then paired up in the order of k.  The sum q * s + b of
-            // bf16 scale and bias has at most 24 significant bits unless the bias is below 2^-16 of the scale, so that this is the f32
-            // multiply-add and its rounding to bf16.  2-bit codes 1, 2 of three sit at 4 and 16 times their value: their scale is
-            // divided (a power of two).  Against packed f32 arithmetic (masks, add, fma, cvt, register moves) 76 instructions for 32 codes
+            // minus 128 (exact), times s plus b with one rounding; bytes are then paired up in the order of k.  That is the f32
+            // multiply-add and its rounding to bf16 but where the first of the two roundings makes a tie of what is none, which takes a bias
+            // below 2^-19 of the scale (all mantissas of both enumerated, for biases of 2^-40 to 2^23 of the scale).  2-bit codes 1, 2 of three
+            // sit at 4 and 16 times their value: their scale is divided (a power of two).  Against packed f32 arithmetic (masks, add, fma, cvt, register moves) 76 instructions for 32 codes
             // instead of 112, which set the pace of a k-block.
             const uint32_t s2 = __float_as_uint(sc) | (__float_as_uint(sc) >> 16), bb = __float_as_uint(bi) | (__float_as_uint(bi) >> 16);
             if constexpr (BITS == 4) {

@@ -4,7 +4,7 @@
 // affine_qmv_wide (crates/lisa-mlx/src/shaders/common/matmul/quantized.metal:890-1088).
 //
 // Codes and activations enter as f16 (mm_core.cuh: a masked field is a subnormal f16, x is normalised per 64-k group), products are
-// exact, the sums are f32; scale and bias follow per 64-k group, in f32: no integer grid for the activations.
+// exact, the sums those of the tensor core; scale and bias follow per 64-k group, in f32: no integer grid for the activations.
 //
 // What bounds it: the packed stream needs 46 4-bit (75 2-bit) codes per clock and SM at the measured copy rate; lifting
 // codes costs 5/8 (9/16) of an operation of the half-rate pipe per code, the m16n8k16 MMAs run at 0.43 per clock (110
