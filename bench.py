@@ -101,11 +101,11 @@ def leg_summary(line):
             "gpu_launches": line.get("gpu_launches"), "roofline": roof}
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum over the algorithmic bytes of the same launches, from the
-# ncu captures (the decode GEMV on 4 layers of the decode stack; the prefill GEMM
+# dram__bytes_read.sum + dram__bytes_write.sum over the algorithmic bytes of the same launches, from
+# ncu captures (profiles/kernels_of_the_cases.md: qmv_dp_kernel<4> on 4 layers of the decode stack, qmm_pair_kernel<4>
 # on 2 layers of the prefill stack).  Traffic grows in proportion to the units processed, so the ratio
 # carries over to a full launch.
-DRAM_TRAFFIC_RATIO = {"decode": 1.005, "prefill": 0.578}
+DRAM_TRAFFIC_RATIO = {"decode": 1.0005, "prefill": 0.606}
 PREFILL_M = 2048
 
 
@@ -676,7 +676,7 @@ def prefill_main(args, torch, dist, stack, rank, local_rank, world, warmup):
             "roofline": {"bound": "tensor", "achieved": per_gpu, "peak": peak, "unit": "TFLOP/s",
                          "frac": per_gpu / peak,
                          "traffic": ratio * stack.prefill_bytes() / launches if ratio else None,
-                         "kernel": "qmm_affine_kernel<4>", "peak_source": src},
+                         "kernel": "qmm_pair_kernel<4>", "peak_source": src},
             "e2e": {"value": world * flops / (e2e_ms * 1e-3) / 1e12, "unit": "TFLOP/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "ms_per_step": e2e_ms},
             "gpu_launches": launches * args.steps, "clocks": clocks, "device_status": ops.device_status(),
