@@ -263,7 +263,7 @@ class DecodeStack:
         self.flags = _cabi.FLAG_PDL if os.environ.get("LISA_BENCH_PDL", "1") != "0" else 0
         if os.environ.get("LISA_BENCH_SIMPLE", "0") == "1":
             self.flags |= _cabi.FLAG_FORCE_QMV_SIMPLE
-        if os.environ.get("LISA_BENCH_TC", "1") == "0":  # the mma.sync kernel instead of the tensor-memory one
+        if os.environ.get("LISA_BENCH_TC", "1") == "0":  # the bf16 mma.sync kernel instead of the default
             self.flags |= _cabi.FLAG_FORCE_QMV
         self.graph = None
         self.siblings = os.environ.get("LISA_BENCH_SIBLINGS", "1") == "1"

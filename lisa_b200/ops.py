@@ -189,7 +189,7 @@ def packed_matmul(fmt, weights: torch.Tensor, input: torch.Tensor, *, workspace:
                   stream=None) -> torch.Tensor:
     """``packed_matvec`` for many tokens with a workspace: products of 32 tokens or more run on the
     tensor cores (operands as hi + lo bf16 planes, f32 accumulate and output, ~1e-4 of the matvec);
-    everything else is the exact matvec."""
+    everything else is the matvec."""
     return _native.packed_matmul(_format_code(fmt), weights, input, workspace, stream)
 
 
