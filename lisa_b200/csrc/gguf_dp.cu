@@ -458,30 +458,39 @@ GdPlan gd_make_plan(int fmt, int64_t zs, int64_t rows, int64_t row_bytes, bool e
     pl.piece = row_bytes % 16 == 0 ? 16 : 4;
     p.tail_pieces = nb % blocks ? static_cast<int>(nb % blocks) * block / pl.piece : 0;
     p.octets = static_cast<int>((rows + 7) / 8);
-    // CTAs of one z: those that fill the SMs once over all z, never more than octets
-    p.ctas = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(p.octets, sm_count() / zs)));
-    p.base = p.octets / p.ctas;
-    p.extra = p.octets % p.ctas;
-    const int per = p.base + (p.extra ? 1 : 0);
-    double best = 1e30;
-    for (int parts = 1; parts <= std::min(p.steps, 64); ++parts) {
-        const int spt = (p.steps + parts - 1) / parts;
-        if ((p.steps + spt - 1) / spt != parts) continue;
-        if (exact && spt != (p.steps + 15) / 16) continue;  // cut by the length of a row alone: a row has the same bits whatever the matrix and the slots
-        const double cost = ((per * parts + kGdWarps - 1) / kGdWarps) * (spt + 0.1) + 0.01 * parts;
-        if (cost < best) {
-            best = cost;
-            p.parts = parts;
-            p.spt = spt;
-        }
-    }
     const int xv = (exact ? 4 : 3) * (fmt == 4 ? 4 : 8), subs = fmt == 4 ? 2 : 8;
     const int64_t fixed = static_cast<int64_t>(p.steps) * (xv * 128 + 8 * subs * 8);
     if (fixed > (1 << 20)) return pl;
     p.ring_at = static_cast<int>((fixed + 127) & ~127);
     p.part_at = p.ring_at + kGdWarps * kGdDepth * 8 * (fmt == 4 ? 320 : 352);
-    const int64_t bytes = p.part_at + static_cast<int64_t>(per) * 8 * p.parts * 4;
-    if (bytes > max_smem_optin() - 2048) return pl;
+    // CTAs of one z: those that fill the SMs once over all z, never more than octets
+    p.ctas = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(p.octets, sm_count() / zs)));
+    int64_t bytes = 0;
+    for (;; p.ctas = std::min(p.octets, 2 * p.ctas)) {
+        p.base = p.octets / p.ctas;
+        p.extra = p.octets % p.ctas;
+        const int per = p.base + (p.extra ? 1 : 0);
+        double best = 1e30;
+        for (int parts = 1; parts <= std::min(p.steps, 64); ++parts) {
+            const int spt = (p.steps + parts - 1) / parts;
+            if ((p.steps + spt - 1) / spt != parts) continue;
+            const double cost = ((per * parts + kGdWarps - 1) / kGdWarps) * (spt + 0.1) + 0.01 * parts;
+            if (cost < best) {
+                best = cost;
+                p.parts = parts;
+                p.spt = spt;
+            }
+        }
+        if (exact) {
+            // Cut by the length of a row alone: a row has the same bits whatever the matrix and the slots.  Rows whose sums of so many parts do not
+            // fit are dealt to more CTAs, so that what fits depends on the length too.
+            p.spt = (p.steps + 15) / 16;
+            p.parts = (p.steps + p.spt - 1) / p.spt;
+        }
+        bytes = p.part_at + static_cast<int64_t>(per) * 8 * p.parts * 4;
+        if (bytes <= max_smem_optin() - 2048) break;
+        if (!exact || p.ctas == p.octets) return pl;
+    }
     pl.smem = static_cast<int>(bytes);
     pl.ok = true;
     return pl;

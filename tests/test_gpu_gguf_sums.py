@@ -65,9 +65,11 @@ def test_bits_of_a_row_do_not_depend_on_the_matrix_or_the_batch(cuda, name, fmt,
         assert torch.equal(ops.packed_matvec(name, w[:2304].contiguous(), x[9:10].contiguous()), full[9:10, :2304])
 
 
-def test_bits_of_an_expert_row_do_not_depend_on_the_slots(cuda):
+# a row's sums of sixteen parts fit a CTA, or not (one CTA per slot: more slots than SMs)
+@pytest.mark.parametrize("rows,k,tokens", [(512, 2304, 20), (8192, 5376, 60)])
+def test_bits_of_an_expert_row_do_not_depend_on_the_slots(cuda, rows, k, tokens):
     rng = np.random.default_rng(5)
-    experts, rows, k, tokens, top_k = 6, 512, 2304, 20, 3
+    experts, top_k = 3, 3
     w = dev_u8(util.gguf_weights(rng, O.Q2_K, rows, k, experts=experts), cuda)
     x = dev_f32(rng.normal(0, 1, size=(tokens, 1, k)).astype(np.float32), cuda)
     ids = torch.from_numpy(rng.integers(0, experts, size=(tokens, top_k)).astype(np.int32)).to(cuda)
