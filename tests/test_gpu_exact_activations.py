@@ -1,6 +1,6 @@
-"""Operators that take the activations as they are -- 8-bit codes, group sizes 32 and 128, the routed block -- on inputs where a coarse grid of
-the activations shows: in every 32 of k one element is `ratio` times the rest, and the weights are zero there.  The default dispatch runs,
-whatever kernel that is."""
+"""Operators that take the activations as they are -- 8-bit codes, group sizes 32 and 128, three to eight rows, the routed block -- on inputs where a
+coarse grid of the activations shows: in every 32 of k one element is `ratio` times the rest, and the weights are zero there.  And the bound of
+the grid where there is one: 2- and 4-bit codes with group size 64 at one and two rows.  The default dispatch runs, whatever kernel that is."""
 import numpy as np
 import pytest
 
@@ -43,6 +43,25 @@ def test_heavy_tails(cuda, bits, gs, n, k, m, ratio):
     terms = np.abs(O.bf16_to_f32(x).astype(np.float64)) @ np.abs(O.affine_dequantize(w, s, b, gs, bits, out_f32=True).astype(np.float64)).T
     # the rounding of the output, and of f32 sums over the terms that are not zero
     assert np.all(np.abs(O.bf16_to_f32(host_bf16_bits(y)) - truth) <= 2.0 ** -8 * np.abs(truth) + 2.0 ** -16 * terms)
+
+
+@pytest.mark.parametrize("bits", [4, 2])
+@pytest.mark.parametrize("n,k", [(264, 1280), (72, 4352)])
+@pytest.mark.parametrize("m", [1, 2, 3, 8])
+@pytest.mark.parametrize("ratio", [2.0 ** 6, 2.0 ** 10])
+def test_heavy_tails_of_group_size_64(cuda, bits, n, k, m, ratio):
+    """One and two rows: an element is off by at most 2^-14 of its group's largest power of two (include/lisa_cuda.h)."""
+    rng = np.random.default_rng(n + k + bits + m)
+    w, s, _ = util.affine_weights(rng, n, k, bits, 64)
+    x, hot = _tails(rng, m, k, ratio)
+    w, b = _without(w, hot, bits), np.zeros_like(s)
+    y = ops.quantized_matmul(dev_bf16(x, cuda), dev_u32(w, cuda), dev_bf16(s, cuda), dev_bf16(b, cuda), True, 64, bits)
+    truth = O.affine_matmul(x, w, s, b, 64, bits, round_weight_bf16=False, f64=True).astype(np.float64)
+    xf = np.abs(O.bf16_to_f32(x).astype(np.float64))
+    wabs = np.abs(O.affine_dequantize(w, s, b, 64, bits, out_f32=True).astype(np.float64))
+    step = 2.0 ** (np.floor(np.log2(xf.reshape(m, k // 64, 64).max(axis=2))) - 14) if m <= 2 else np.zeros((m, k // 64))
+    bound = np.einsum("ngk,mg->mn", wabs.reshape(n, k // 64, 64), step) + 2.0 ** -8 * np.abs(truth) + 2.0 ** -16 * (xf @ wabs.T)
+    assert np.all(np.abs(O.bf16_to_f32(host_bf16_bits(y)) - truth) <= bound)
 
 
 @pytest.mark.parametrize("scale", [2.0 ** -100, 2.0 ** -118])
